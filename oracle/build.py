@@ -32,7 +32,7 @@ def build_oracle(quiet: bool = True) -> str:
 def build_reference(reference: str = DEFAULT_REFERENCE, quiet: bool = True) -> str | None:
     """Builds oracle/_ref/libref_glsl.so, libref_tes.so, libref_skin.so and
     libref_marschner_{m,n}.so if the reference tree is present."""
-    if not os.path.isdir(reference):
+    if not os.path.isdir(os.path.join(reference, "src", "shaders")):
         return None
     sys.path.insert(0, os.path.join(HERE, "ref_glsl"))
     try:
