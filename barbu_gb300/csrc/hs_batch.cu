@@ -237,7 +237,7 @@ __global__ void __launch_bounds__(K * 32, 16 / K)
       __syncthreads();
     }
     const SphereSet S{e.fc.spheres, e.fc.r2, e.fc.adj, e.fc.nspheres};
-    tile_frame_lanes<K, kCachedSpheres, false, FAST>(e.fc, S, e.view, strand0 / kWarp, s_p, s_v, s_ts);
+    tile_frame_lanes<K, FAST>(e.fc, S, e.view, strand0 / kWarp, s_p, s_v, s_ts);
     __syncthreads();  // the next tile rewrites s_next, the entry and the state
   }
 }

@@ -127,9 +127,8 @@ __global__ void __launch_bounds__(kStreamBlock) k_step_stream(GroomView g, Frame
 // TMEM velocity slots).
 constexpr int kTmemBlock = 128;
 
-// CACHED: pushes from the register sphere cache (hs_stream.cuh, push_seg),
-// for grooms among many spheres.
-template <bool REF, bool CACHED, bool FAST>
+// MANY: the push-out's form for grooms among many spheres (push_seg).
+template <bool REF, bool MANY, bool FAST>
 __global__ void __launch_bounds__(kTmemBlock) k_step_stream_tmem(GroomView g, FrameConst fc) {
   extern __shared__ float4 s_pos[];  // positions, compact: float2 (x, y) then float z, each [npoints][kTmemBlock]
   __shared__ float4 s_c[HS_MAX_SPHERES];
@@ -154,7 +153,7 @@ __global__ void __launch_bounds__(kTmemBlock) k_step_stream_tmem(GroomView g, Fr
   float2* xy = reinterpret_cast<float2*>(s_pos);
   float* z = reinterpret_cast<float*>(xy + g.npoints * kTmemBlock);
   const XShared3 X{xy + threadIdx.x, z + threadIdx.x, kTmemBlock};
-  strand_frame_stream<REF, XShared3, VTmem, 8, true, CACHED, FAST>(fc, S, g, s, s < g.nstrands, X, V);
+  strand_frame_stream<REF, XShared3, VTmem, 8, true, MANY, FAST>(fc, S, g, s, s < g.nstrands, X, V);
   tmem::fence_before_sync();
   __syncthreads();
   tmem::fence_after_sync();
@@ -174,40 +173,36 @@ size_t tmem_step_smem(uint32_t npoints) {
   return std::max(need, per_block > fixed ? per_block - fixed : need);
 }
 
+// Spheres of a groom up to which its strands reach few of them, and the
+// push-out goes through all of those (measured at 7 and 16: push_seg).
+constexpr int kFewSpheres = 8;
+
+using TmemStep = void (*)(GroomView, FrameConst);
+TmemStep dftl_step_tmem(bool many, bool fast) {
+  if (many) return fast ? k_step_stream_tmem<false, true, true> : k_step_stream_tmem<false, true, false>;
+  return fast ? k_step_stream_tmem<false, false, true> : k_step_stream_tmem<false, false, false>;
+}
+
 cudaError_t launch_step_stream_tmem(const GroomView& g, const FrameConst& fc, cudaStream_t st) {
   const unsigned grid = (g.nstrands + kTmemBlock - 1) / kTmemBlock;
   const size_t smem = tmem_step_smem(g.npoints);
   static std::atomic<uint64_t> optin{0};
   once_per_device(optin, [] {
     const int bytes = 200 * 1024;
+    for (const bool fast : {false, true})
+      for (const bool many : {false, true})
+        cudaFuncSetAttribute(dftl_step_tmem(many, fast), cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     cudaFuncSetAttribute(k_step_stream_tmem<true, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    cudaFuncSetAttribute(k_step_stream_tmem<false, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    cudaFuncSetAttribute(k_step_stream_tmem<false, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    cudaFuncSetAttribute(k_step_stream_tmem<false, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    cudaFuncSetAttribute(k_step_stream_tmem<false, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
   });
-  // Grooms among many spheres push at most points: the register-cached
-  // push pays there (skinned groom, 32 spheres: 5.53 -> 4.60 ms a frame)
-  // and costs elsewhere in instruction-cache space (large groom, 16
-  // spheres: 0.364 -> 0.462 ms).
-  const bool cached = fc.nspheres > 16;
-  const bool fast = fast_frame(fc);
-  if (fc.mode == HS_MODE_REFERENCE) {
+  if (fc.mode == HS_MODE_REFERENCE)
     return launch_overlapped(k_step_stream_tmem<true, false, false>, grid, kTmemBlock, smem, st, g, fc);
-  } else if (cached) {
-    if (fast) return launch_overlapped(k_step_stream_tmem<false, true, true>, grid, kTmemBlock, smem, st, g, fc);
-    return launch_overlapped(k_step_stream_tmem<false, true, false>, grid, kTmemBlock, smem, st, g, fc);
-  } else {
-    if (fast) return launch_overlapped(k_step_stream_tmem<false, false, true>, grid, kTmemBlock, smem, st, g, fc);
-    return launch_overlapped(k_step_stream_tmem<false, false, false>, grid, kTmemBlock, smem, st, g, fc);
-  }
+  return launch_overlapped(dftl_step_tmem(fc.nspheres > kFewSpheres, fast_frame(fc)), grid, kTmemBlock, smem, st, g, fc);
 }
 
 // Lane groups (hs_lanes.cuh): a block of K warps per 32-strand tile, the
 // tile's starting state in shared memory ([npoints][32] positions, then
-// velocities). Register cap 128 (16 warps a SM). CACHED: as the
-// tensor-memory step (grooms among many spheres).
-template <int K, bool CACHED, bool FAST>
+// velocities). Register cap 128 (16 warps a SM).
+template <int K, bool FAST>
 __global__ void __launch_bounds__(K * 32, 16 / K) k_step_lanes(GroomView g, FrameConst fc) {
   extern __shared__ float4 s_state[];
   __shared__ float4 s_c[HS_MAX_SPHERES];
@@ -217,7 +212,7 @@ __global__ void __launch_bounds__(K * 32, 16 / K) k_step_lanes(GroomView g, Fram
   frame_release();
   const SphereSet S = stage_spheres(fc, s_c, s_r2, s_adj);
   frame_acquire();
-  tile_frame_lanes<K, 8, CACHED, FAST>(fc, S, g, blockIdx.x, s_state, s_state + g.npoints * 32, s_ts);
+  tile_frame_lanes<K, FAST>(fc, S, g, blockIdx.x, s_state, s_state + g.npoints * 32, s_ts);
 }
 
 template <int K>
@@ -227,17 +222,12 @@ cudaError_t launch_step_lanes_k(const GroomView& g, const FrameConst& fc, cudaSt
   static std::atomic<uint64_t> optin{0};
   once_per_device(optin, [] {
     const int bytes = 2 * static_cast<int>(sizeof(float4)) * 32 * HS_MAX_POINTS_PER_STRAND;
-    cudaFuncSetAttribute(k_step_lanes<K, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    cudaFuncSetAttribute(k_step_lanes<K, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    cudaFuncSetAttribute(k_step_lanes<K, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    cudaFuncSetAttribute(k_step_lanes<K, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    cudaFuncSetAttribute(k_step_lanes<K, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    cudaFuncSetAttribute(k_step_lanes<K, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
   });
-  const bool cached = fc.nspheres > 16, fast = fast_frame(fc);
   const unsigned block = K * 32;
-  if (cached && fast) return launch_overlapped(k_step_lanes<K, true, true>, grid, block, smem, st, g, fc);
-  if (cached) return launch_overlapped(k_step_lanes<K, true, false>, grid, block, smem, st, g, fc);
-  if (fast) return launch_overlapped(k_step_lanes<K, false, true>, grid, block, smem, st, g, fc);
-  return launch_overlapped(k_step_lanes<K, false, false>, grid, block, smem, st, g, fc);
+  if (fast_frame(fc)) return launch_overlapped(k_step_lanes<K, true>, grid, block, smem, st, g, fc);
+  return launch_overlapped(k_step_lanes<K, false>, grid, block, smem, st, g, fc);
 }
 
 cudaError_t launch_step_lanes(const GroomView& g, const FrameConst& fc, cudaStream_t st) {

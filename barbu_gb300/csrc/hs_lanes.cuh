@@ -26,8 +26,8 @@
 // The arithmetic of every point and substep is that of
 // substep_single_pass_seg, so the frames are bit-identical to the
 // thread-per-strand kernels'. Which points test the spheres (jmin, per
-// strand here) and how (the cache width) change no result: a point that
-// cannot reach a sphere is never pushed.
+// strand here) changes no result: a point that cannot reach a sphere is
+// never pushed.
 #pragma once
 
 #include "hs_stream.cuh"
@@ -55,17 +55,15 @@ __device__ __forceinline__ void load_start(bool take, const float4* sp, const fl
       : "memory");
 }
 
-// The wavefront of one strand's substeps (see the header). NC: sphere
-// slots tested; CACHED: push from the register cache (push_seg). s_p holds
+// The wavefront of one strand's substeps (see the header). s_p holds
 // the strand's starting segments (point 0: its world position) with the
 // rest lengths in w, s_v its velocities, [point][32] at column c. The lane
 // of the last substep stores the finished points and adds them to `ts`.
-template <int K, int NC, bool CACHED, bool FAST, int M>
-__device__ __forceinline__ void lanes_pass(const FrameConst& fc, const StrandConsts& Kc, const SphereCache<M>& C,
+template <int K, bool FAST, int NF>
+__device__ __forceinline__ void lanes_pass(const FrameConst& fc, const StrandConsts& Kc, const SphereFilter<NF>& F,
                                            const SphereSet& S, const GroomView& g, uint32_t s, bool active, int c,
                                            int k, int n, int jmin, V3 x0_start, V3 target, float rest0,
                                            const float4* s_p, const float4* s_v, TileStats& ts) {
-  constexpr bool kCached = CACHED && M > kCachedSpheres;
   const V3 zero = v3(0.0f, 0.0f, 0.0f);
   const int nsub = fc.substeps;
   const bool worker = k < nsub;
@@ -111,8 +109,7 @@ __device__ __forceinline__ void lanes_pass(const FrameConst& fc, const StrandCon
     const V3 w_i = add(w_prev, sn);
     // Finish point j - 1 (2 <= j <= n).
     const bool fin = worker && j >= 2 && j <= n;
-    if (fin && j - 1 >= jmin && tests<NC>(C, w_prev))
-      push_seg<kCached, NC, FAST>(C, S, w_prev, D_prev, s_prev, sn, tip);
+    if (fin && j - 1 >= jmin && flagged(F, w_prev)) push_seg<false, FAST>(F, S, w_prev, D_prev, s_prev, sn, tip);
     const V3 vel = vel_of(Kc, tip ? D_prev : fmas(Kc.neg_damping, e, D_prev));
     if (writer && fin) {
       wout = add(wout, s_prev);
@@ -154,7 +151,7 @@ __device__ __forceinline__ void lanes_pass(const FrameConst& fc, const StrandCon
 // warp w takes strands [w 32/K, (w + 1) 32/K) of the tile, lane l strand
 // l / K as substep lane l % K). s_p, s_v: [n][32] float4 each, the tile's
 // starting state; s_ts: 32 TileStats. Every thread of the block calls it.
-template <int K, int M, bool CACHED, bool FAST>
+template <int K, bool FAST>
 __device__ __forceinline__ void tile_frame_lanes(const FrameConst& fc, const SphereSet& S, const GroomView& g,
                                                  uint32_t tile, float4* s_p, float4* s_v, TileStats* s_ts) {
   static_assert(K == 2 || K == 4 || K == 8 || K == 16, "lane groups of 2, 4, 8 or 16");
@@ -209,28 +206,24 @@ __device__ __forceinline__ void tile_frame_lanes(const FrameConst& fc, const Sph
   // that can touch one (strand_frame_stream), per strand.
   uint32_t reach = 0u;
   int jmin = n;
+  float far = 0.0f;
   if (S.n > 0 && active) {
-    const V3 root_delta = sub(target, x0_start);
-    const V3 mid = v3(0.5f * (x0_start.x + target.x), 0.5f * (x0_start.y + target.y), 0.5f * (x0_start.z + target.z));
-    const float half_path = 0.5f * sqrtf(root_delta.x * root_delta.x + root_delta.y * root_delta.y +
-                                         root_delta.z * root_delta.z);
-    reach = overlap_closure(S, near_spheres(S, mid, Rlen + half_path));
-    const float thr = reach_threshold(S, mid, Rlen + half_path, half_path);
-    float Rj = 0.0f;
-    for (int i = 1; i < n; ++i) {
-      Rj += fabsf(fc.length_scale * s_p[i * 32 + c].w);
-      if (jmin == n && Rj >= thr) jmin = i;
+    const StrandBall ball(x0_start, target, Rlen);
+    const SphereReach q = sphere_reach(S, ball);
+    reach = overlap_closure(S, q.near);
+    far = ball.far();
+    if (reach) {
+      float Rj = 0.0f;
+      for (int i = 1; i < n; ++i) {
+        Rj += fabsf(fc.length_scale * s_p[i * 32 + c].w);
+        if (jmin == n && Rj >= q.threshold) jmin = i;
+      }
     }
   }
-  const SphereCache<M> C = cache_spheres<M>(S, reach);
+  const SphereFilter<8> F = filter_spheres<8>(S, reach, far);
   TileStats ts;
   ts.init();
-  const int warp_cached = __reduce_max_sync(0xffffffffu, C.ncached);
-  if (M > kCachedSpheres && warp_cached > kCachedSpheres)
-    lanes_pass<K, M, CACHED, FAST>(fc, Kc, C, S, g, s, active, c, k, n, jmin, x0_start, target, rest0, s_p, s_v, ts);
-  else
-    lanes_pass<K, kCachedSpheres, CACHED, FAST>(fc, Kc, C, S, g, s, active, c, k, n, jmin, x0_start, target, rest0,
-                                                s_p, s_v, ts);
+  lanes_pass<K, FAST>(fc, Kc, F, S, g, s, active, c, k, n, jmin, x0_start, target, rest0, s_p, s_v, ts);
 
   // Tile statistics: the strands' own (from their last substep's lane, in
   // point order), reduced by one warp as the thread-per-strand kernels do.

@@ -70,6 +70,12 @@ __device__ __forceinline__ float4 with_rest(float4 x, float4 v) {
   if constexpr (XS::kRestInV) return make_float4(x.x, x.y, x.z, v.w);
   else return x;
 }
+// The rest length of point i alone.
+template <typename XS, typename VS>
+__device__ __forceinline__ float rest_of(const XS& X, const VS& V, int i) {
+  if constexpr (XS::kRestInV) return V.load_w(i);
+  else return X.load(i).w;
+}
 // The w a velocity slot stores: the rest length where it lives there.
 template <typename XS>
 __device__ __forceinline__ float vel_w(float rest) {
@@ -77,9 +83,10 @@ __device__ __forceinline__ float vel_w(float rest) {
   else return 0.0f;
 }
 
-// Up to M of the warp's reachable spheres sit in registers; the rest are
-// read from shared memory. kCachedSpheres is the width of the batched
-// kernels' cache; the plain step also has an 8-wide one (strand_frame_stream).
+// Reference mode: up to M of a strand's reachable spheres sit in registers;
+// the rest are read from shared memory. kCachedSpheres is the width of the
+// batched kernels' cache; the plain step also has an 8-wide one
+// (strand_frame_stream). The DFTL passes have a filter (SphereFilter).
 constexpr int kCachedSpheres = 4;
 
 template <int M>
@@ -171,18 +178,18 @@ __device__ __forceinline__ bool tests(const SphereCache<M>& C, V3 p) {
 // The exact in-order push-out (rare), kept inline: an out-of-line call
 // would take the addresses of the callers' per-lane arrays and move them
 // to local memory. True if any sphere pushed the point.
-template <bool REF, int NC, bool FAST = false, int M>
+template <bool REF, int NC, int M>
 __device__ __forceinline__ bool push_all(const SphereCache<M>& C, const SphereSet& S, V3& p, V3& v) {
   bool pushed = false;
 #pragma unroll
   for (int q = 0; q < M; ++q)
-    if (q < C.ncached) pushed |= push_out<REF, FAST>(v3(C.cx[q], C.cy[q], C.cz[q]), C.r[q], C.r2[q], p, v);
+    if (q < C.ncached) pushed |= push_out<REF>(v3(C.cx[q], C.cy[q], C.cz[q]), C.r[q], C.r2[q], p, v);
   uint32_t more = C.rest;
   while (more) {
     const int k = __ffs(more) - 1;
     more &= more - 1u;
     const float4 c = S.c[k];
-    pushed |= push_out<REF, FAST>(v3(c.x, c.y, c.z), c.w, S.r2[k], p, v);
+    pushed |= push_out<REF>(v3(c.x, c.y, c.z), c.w, S.r2[k], p, v);
   }
   return pushed;
 }
@@ -371,44 +378,218 @@ __device__ __forceinline__ void link_seg(const StrandConsts& K, V3 d, float rest
   e = sub(sn, d);
 }
 
-// Push-out of one point against the spheres of `reach`, in index order,
-// read from shared memory: the exact in-order push of push_all (the cached
-// spheres are copies of the same entries, taken in index order), as one
-// small loop rather than push_all's unrolled cache.
-struct Pushed {
-  V3 p;
-  bool pushed;
+// ---- spheres of the DFTL passes ------------------------------------------
+//
+// A point is first tested against a conservative filter, and only a flagged
+// one runs the exact in-order push-out (push_seg). The filter holds, of the
+// spheres the strand can reach, up to NF as (-2c, |c|^2 - r^2 - margin): a
+// point p inside sphere k has dot(-2c, p) + (|c|^2 - r^2 - margin) <=
+// -|p|^2. That is three fused multiply-adds a sphere, where the exact test
+// takes six operations and a comparison, and its slots 2-3 and 4-7 are
+// skipped by warps whose strands reach no more than two or four spheres
+// (two thirds of the 64-groom workload's warps reach at most two). More than
+// NF spheres: the last slot is a ball around the rest, which flags points it
+// need not. Measured against exact tests of four cached spheres, which sent
+// every point of a strand with more to the push-out, and the set-up below
+// done with IEEE divisions and square roots in two loops over the spheres:
+// 64-groom frame 938 -> 773 us, 262,144 x 32 groom 284 -> 242 us (EXACT),
+// 251 -> 218 us (FAST).
+//
+// The margin. With u = 2^-24, the exact test dot(p - c, p - c) < fl(r^2)
+// in FP32 implies |p - c|^2 < r^2 (1 + 8u); the rounding of the filter's
+// sums (three terms each) is below 9u ((|p| + |c|)^2 + r^2): together less
+// than 17u = 1.02e-6 times that, and the margin is 1.25e-6 times it (at
+// 4e-6 the points resting near a surface were flagged, and more warps took
+// the push-out). |p| is bounded by the ball the strand stays in during the
+// frame (near_spheres, its margins included).
+template <int NF>
+struct SphereFilter {
+  float cx[NF], cy[NF], cz[NF], k[NF];
+  uint32_t reach;  // the strand's reachable spheres
+  bool many;       // a strand of the warp reaches more than two
+  bool most;       // more than four
 };
-template <bool FAST = false>
-__device__ __forceinline__ Pushed push_mask(uint32_t reach, const float4* c, const float* r2, V3 p) {
-  bool pushed = false;
-  V3 unused = v3(0.0f, 0.0f, 0.0f);
-  while (reach) {
-    const int k = __ffs(reach) - 1;
-    reach &= reach - 1u;
-    const float4 ck = c[k];
-    pushed |= push_out<false, FAST>(v3(ck.x, ck.y, ck.z), ck.w, r2[k], p, unused);
-  }
-  return Pushed{p, pushed};
+
+// Square root to a few ulp, for distances that are compared with a margin
+// of 1e-3.
+__device__ __forceinline__ float sqrt_near(float x) {
+  float y;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
 }
-// Push-out of point j at its chain position w: a push by g moves D_j and
-// s_j by +g and the next segment by -g (none at the tip). CACHED: the
-// in-order push from the register cache (push_all, unrolled over its
-// slots: more code, fewer instructions a push), for grooms among many
-// spheres that push at most points; else the small loop of push_mask.
-// FAST: the push-out of the FAST contract (push_out).
-template <bool CACHED, int NC, bool FAST = false, int M>
-__device__ __forceinline__ void push_seg(const SphereCache<M>& C, const SphereSet& S, V3 w, V3& D, V3& s,
-                                         V3& s_next, bool tip) {
-  Pushed r{w, false};
-  if constexpr (CACHED) {
-    V3 unused = v3(0.0f, 0.0f, 0.0f);
-    r.pushed = push_all<false, NC, FAST>(C, S, r.p, unused);
-  } else {
-    r = push_mask<FAST>(C.reach, S.c, S.r2, w);
+
+// The ball a strand stays in during the frame: the root's path about its
+// midpoint, and the links' total length R beyond it.
+struct StrandBall {
+  V3 mid;
+  float half_path, radius;
+  __device__ __forceinline__ StrandBall(V3 x0, V3 target, float R) {
+    const float dx = target.x - x0.x, dy = target.y - x0.y, dz = target.z - x0.z;
+    mid = v3(0.5f * (x0.x + target.x), 0.5f * (x0.y + target.y), 0.5f * (x0.z + target.z));
+    half_path = 0.5f * sqrt_near(dx * dx + dy * dy + dz * dz);
+    radius = R + half_path;
   }
-  if (r.pushed) {
-    const V3 g = sub(r.p, w);
+  // The largest |p| of a point in it, with near_spheres' margins.
+  __device__ __forceinline__ float far() const {
+    return (sqrt_near(mid.x * mid.x + mid.y * mid.y + mid.z * mid.z) + radius) * 1.002f + 1.0e-3f;
+  }
+};
+
+// near_spheres (hs_step.cuh) of one strand, and the smallest summed link
+// length at which a point of it may touch a sphere: the distance from `mid`
+// to the sphere's surface less the root's half path, with the same margins.
+// A point whose links from the root sum to less cannot be inside any sphere
+// this frame.
+struct SphereReach {
+  uint32_t near;
+  float threshold;
+};
+__device__ __forceinline__ SphereReach sphere_reach(const SphereSet& S, const StrandBall& b) {
+  const float mag = fmaxf(fmaxf(fabsf(b.mid.x), fabsf(b.mid.y)), fmaxf(fabsf(b.mid.z), b.radius)) + 1.0f;
+  const float slack = mag * 1.0e-4f;
+  SphereReach o{0u, 3.0e38f};
+#pragma unroll 2
+  for (int k = 0; k < S.n; ++k) {
+    const float4 c = S.c[k];
+    const float dx = c.x - b.mid.x, dy = c.y - b.mid.y, dz = c.z - b.mid.z;
+    const float d2 = dx * dx + dy * dy + dz * dz;
+    const float reach = (c.w + b.radius) * 1.001f + slack;
+    if (d2 < reach * reach) o.near |= 1u << k;
+    o.threshold = fminf(o.threshold, (sqrt_near(d2) - slack) * 0.999f - c.w - b.half_path);
+  }
+  return o;
+}
+
+// far: the largest |p| of the strand's points during the frame. Every lane
+// of the warp calls it. Slots that no strand of the warp fills are left out
+// (flagged does not read them).
+template <int NF>
+__device__ __forceinline__ SphereFilter<NF> filter_spheres(const SphereSet& S, uint32_t reach, float far) {
+  SphereFilter<NF> F;
+  F.reach = reach;
+  F.many = __any_sync(0xffffffffu, __popc(reach) > 2);
+  F.most = NF > 4 && __any_sync(0xffffffffu, __popc(reach) > 4);
+#pragma unroll
+  for (int q = 0; q < NF; ++q) {
+    float cx = 0.0f, cy = 0.0f, cz = 0.0f, kk = __int_as_float(0x7f800000);  // no sphere: never flagged
+    if ((q < 2 || (q < 4 ? F.many : F.most)) && reach) {
+      const int i = __ffs(reach) - 1;
+      const uint32_t more = reach & (reach - 1u);
+      const float4 c = S.c[i];
+      cx = c.x;
+      cy = c.y;
+      cz = c.z;
+      float r2 = S.r2[i];
+      if (q == NF - 1 && more) {
+        // A ball around the remaining spheres, centred about their mean.
+        float cnt = 1.0f;
+        for (uint32_t m = more; m; m &= m - 1u) {
+          const float4 d = S.c[__ffs(m) - 1];
+          cx += d.x;
+          cy += d.y;
+          cz += d.z;
+          cnt += 1.0f;
+        }
+        cnt = __fdividef(1.0f, cnt);
+        cx *= cnt;
+        cy *= cnt;
+        cz *= cnt;
+        float rr = 0.0f;
+        for (uint32_t m = reach; m; m &= m - 1u) {
+          const float4 d = S.c[__ffs(m) - 1];
+          const float dx = d.x - cx, dy = d.y - cy, dz = d.z - cz;
+          rr = fmaxf(rr, sqrt_near(dx * dx + dy * dy + dz * dz) + d.w);
+        }
+        rr = rr * 1.0001f + 1.0e-5f * (fabsf(cx) + fabsf(cy) + fabsf(cz));
+        r2 = rr * rr;
+      }
+      reach = more;
+      const float c2 = cx * cx + cy * cy + cz * cz;
+      const float big = far + sqrt_near(c2) * 1.0001f;
+      const float size = big * big + r2;
+      // Coordinates too large for the sums: every point is flagged.
+      kk = size < 1.0e30f ? (c2 - r2) - (1.25e-6f * size + 1.0e-30f) : __int_as_float(0xff800000);
+    }
+    F.cx[q] = -2.0f * cx;
+    F.cy[q] = -2.0f * cy;
+    F.cz[q] = -2.0f * cz;
+    F.k[q] = kk;
+  }
+  return F;
+}
+
+template <int NF>
+__device__ __forceinline__ float filter_value(const SphereFilter<NF>& F, int q, V3 w) {
+  return __fmaf_rn(F.cx[q], w.x, __fmaf_rn(F.cy[q], w.y, __fmaf_rn(F.cz[q], w.z, F.k[q])));
+}
+
+// Whether a point may be inside a sphere. (Overflow: an infinite |p|^2 flags
+// nothing a finite slot did not, and such a point is in no sphere.)
+template <int NF>
+__device__ __forceinline__ bool flagged(const SphereFilter<NF>& F, V3 w) {
+  float m = fminf(filter_value(F, 0, w), filter_value(F, 1, w));
+  if (F.many) {
+#pragma unroll
+    for (int q = 2; q < 4; ++q) m = fminf(m, filter_value(F, q, w));
+    if (NF > 4 && F.most) {
+#pragma unroll
+      for (int q = 4; q < NF; ++q) m = fminf(m, filter_value(F, q, w));
+    }
+  }
+  return m <= -dot(w, w);
+}
+
+// The exact in-order push-out (push_out) of point j at its chain position w,
+// against the strand's reachable spheres in index order, read from shared
+// memory. A push by g moves D_j and s_j by +g and the next segment by -g
+// (none at the tip).
+//
+// A strand in contact waits for this path at every point-substep, so it has
+// no branch around the push: with one, a frame of 50,021 x 23 strands among
+// 7 spheres takes 50.6 instead of 49.6 us. PICK, for grooms among many
+// spheres: warps whose strands reach more than two go through the spheres
+// the point is flagged for alone, and after a push also through the later
+// ones that overlap the pushing sphere (the point, on its surface, can be in
+// no other). 262,144 x 32 strands among 16 spheres: 241 -> 231 us a frame
+// (EXACT), 215 -> 211 us (FAST); the code is larger, which costs the
+// batched kernel more than it saves (64 grooms: 782 -> 824 us) and grooms
+// among few spheres (the 7 above: 49.6 -> 52.1 us).
+template <bool PICK, bool FAST, int NF>
+__device__ __forceinline__ void push_seg(const SphereFilter<NF>& F, const SphereSet& S, V3 w, V3& D, V3& s, V3& s_next,
+                                         bool tip) {
+  uint32_t todo = F.reach;
+  if (PICK && F.many) {
+    const float w2 = dot(w, w);
+    uint32_t left = F.reach;
+    todo = 0u;
+#pragma unroll
+    for (int q = 0; q < NF; ++q) {
+      if (q < 4 || F.most) {
+        const uint32_t low = q == NF - 1 ? left : left & (0u - left);
+        if (filter_value(F, q, w) <= -w2) todo |= low;
+        left ^= low;
+      }
+    }
+  }
+  V3 p = w;
+  bool pushed = false;
+  while (todo) {
+    const int k = __ffs(todo) - 1;
+    todo &= todo - 1u;
+    const float4 c = S.c[k];
+    const V3 cc = v3(c.x, c.y, c.z);
+    const V3 d = sub(p, cc);
+    const float d2 = dot(d, d);
+    const bool hit = d2 < S.r2[k];
+    const V3 u = mul(d, FAST ? rsqrt_fast(d2) : inversesqrt(d2));
+    const bool off = d2 > 0.0f;  // not at the centre
+    const V3 q = add(cc, mul(c.w, v3(off ? u.x : 0.0f, off ? u.y : 1.0f, off ? u.z : 0.0f)));
+    p = v3(hit ? q.x : p.x, hit ? q.y : p.y, hit ? q.z : p.z);
+    pushed |= hit;
+    if (PICK) todo |= hit ? S.adj[k] & F.reach & (0xfffffffeu << k) : 0u;
+  }
+  if (pushed) {
+    const V3 g = sub(p, w);
     D = add(D, g);
     s = add(s, g);
     if (!tip) s_next = sub(s_next, g);
@@ -419,10 +600,10 @@ __device__ __forceinline__ void push_seg(const SphereCache<M>& C, const SphereSe
 // (a_cur = s_i + D_i, dp_cur, rest_cur), loads point i + 1, runs link i,
 // finishes point i - 1, testing it against the spheres if TEST and
 // i - 1 >= jmin.
-template <bool TEST, bool CACHED, int NC, bool FAST, typename XS, typename VS, int M>
+template <bool TEST, bool PICK, bool FAST, typename XS, typename VS, int NF>
 struct SegPass {
   const StrandConsts& K;
-  const SphereCache<M>& C;
+  const SphereFilter<NF>& F;
   const SphereSet& S;
   const XS& X;
   const VS& V;
@@ -436,18 +617,16 @@ struct SegPass {
     if constexpr (VS::kPrefetch) {
       vn = V.complete(pend);
       if (i + 2 < n) pend = V.issue(i + 2);
-    } else {
-      vn = V.load(i + 1);
     }
-    const float4 xn = with_rest<XS>(xr, vn);
-    const V3 dp_next = disp(K, vn);
-    const V3 a_next = add(xyz(xn), dp_next);
+    else vn = V.load(i + 1);
     V3 sn, e;
     link_seg<FAST>(K, sub(a_cur, D_prev), rest_cur, sn, e);
     const V3 D_i = add(dp_cur, e);
     const V3 w_i = add(w_prev, sn);
-    if (TEST && i - 1 >= jmin && tests<NC>(C, w_prev))
-      push_seg<CACHED, NC, FAST>(C, S, w_prev, D_prev, s_prev, sn, false);
+    if (TEST && i - 1 >= jmin && flagged(F, w_prev)) push_seg<PICK, FAST>(F, S, w_prev, D_prev, s_prev, sn, false);
+    const float4 xn = with_rest<XS>(xr, vn);
+    const V3 dp_next = disp(K, vn);
+    const V3 a_next = add(xyz(xn), dp_next);
     X.store(i - 1, f4(s_prev, rest_prev));
     V.store(i - 1, f4(vel_of(K, fmas(K.neg_damping, e, D_prev)), vel_w<XS>(rest_prev)));
     s_prev = sn;
@@ -468,14 +647,12 @@ struct SegPass {
 // cannot reach a sphere this frame (strand_frame_stream) and skip the
 // tests. Measured code shapes (the hot loop must stay in the instruction
 // cache): SPLIT, a loop without tests up to jmin then one with them, else
-// one loop with the jmin check; CACHED (8-wide cache only): the push from
-// the register cache (push_seg).
-template <int NC, bool SPLIT, bool CACHED, bool FAST, typename XS, typename VS, int M>
-__device__ __forceinline__ void substep_single_pass_seg(const StrandConsts& K, const SphereCache<M>& C,
+// one loop with the jmin check.
+template <bool SPLIT, bool PICK, bool FAST, typename XS, typename VS, int NF>
+__device__ __forceinline__ void substep_single_pass_seg(const StrandConsts& K, const SphereFilter<NF>& F,
                                                         const SphereSet& S, int n, int jmin, V3 D0, V3 R,
                                                         const XS& X, const VS& V) {
   constexpr bool kSplit = SPLIT;
-  constexpr bool kCached = CACHED && M > kCachedSpheres;
   // Link 1.
   const float4 v1 = V.load(1);
   const float4 x1 = with_rest<XS>(X.load(1), v1);
@@ -490,8 +667,8 @@ __device__ __forceinline__ void substep_single_pass_seg(const StrandConsts& K, c
     const float4 v2 = V.load(2);
     const float4 x2 = with_rest<XS>(X.load(2), v2);
     const V3 dp2 = disp(K, v2);
-    SegPass<!kSplit, kCached, NC, FAST, XS, VS, M> A{K, C, S, X, V, n, jmin, D_prev, w_prev, s_prev,
-                                               add(xyz(x2), dp2), dp2, rest_prev, x2.w, {}};
+    SegPass<!kSplit, PICK, FAST, XS, VS, NF> A{K,      F,      S,      X,      V,   n, jmin, D_prev, w_prev, s_prev, add(xyz(x2), dp2),
+                                     dp2, rest_prev, x2.w, {}};
     if constexpr (VS::kPrefetch) {
       if (n > 3) A.pend = V.issue(3);
     }
@@ -504,8 +681,8 @@ __device__ __forceinline__ void substep_single_pass_seg(const StrandConsts& K, c
 #pragma unroll 2
       for (; i < ia; ++i) A.step(i);
     }
-    SegPass<true, kCached, NC, FAST, XS, VS, M> B{K, C, S, X, V, n, jmin, A.D_prev, A.w_prev, A.s_prev, A.a_cur,
-                                            A.dp_cur, A.rest_prev, A.rest_cur, A.pend};
+    SegPass<true, PICK, FAST, XS, VS, NF> B{K,        F,        S,           X,          V,     n, jmin, A.D_prev, A.w_prev, A.s_prev,
+                                  A.a_cur, A.dp_cur, A.rest_prev, A.rest_cur, A.pend};
 #pragma unroll 2
     for (; i < n - 1; ++i) B.step(i);
     // Link n-1 and point n-2.
@@ -514,8 +691,7 @@ __device__ __forceinline__ void substep_single_pass_seg(const StrandConsts& K, c
     const V3 w_i = add(B.w_prev, sn);
     D_prev = B.D_prev;
     s_prev = B.s_prev;
-    if (n - 2 >= jmin && tests<NC>(C, B.w_prev))
-      push_seg<kCached, NC, FAST>(C, S, B.w_prev, D_prev, s_prev, sn, false);
+    if (n - 2 >= jmin && flagged(F, B.w_prev)) push_seg<PICK, FAST>(F, S, B.w_prev, D_prev, s_prev, sn, false);
     X.store(n - 2, f4(s_prev, B.rest_prev));
     V.store(n - 2, f4(vel_of(K, fmas(K.neg_damping, e, D_prev)), vel_w<XS>(B.rest_prev)));
     s_prev = sn;
@@ -524,7 +700,7 @@ __device__ __forceinline__ void substep_single_pass_seg(const StrandConsts& K, c
     rest_prev = B.rest_cur;
   }
   // The tip: no next correction, v = D / h.
-  if (n - 1 >= jmin && tests<NC>(C, w_prev)) push_seg<kCached, NC, FAST>(C, S, w_prev, D_prev, s_prev, sn, true);
+  if (n - 1 >= jmin && flagged(F, w_prev)) push_seg<PICK, FAST>(F, S, w_prev, D_prev, s_prev, sn, true);
   X.store(n - 1, f4(s_prev, rest_prev));
   V.store(n - 1, f4(vel_of(K, D_prev), vel_w<XS>(rest_prev)));
 }
@@ -534,10 +710,10 @@ __device__ __forceinline__ void substep_single_pass_seg(const StrandConsts& K, c
 // iteration's link is d = (s_i + D_i) - D_{i-1} (as in the single pass),
 // later ones d = s_i - e_{i-1} (e: that iteration's correction of the
 // leader); the last pass forms the velocities.
-template <int NC, bool FAST, typename XS, typename VS, int M>
-__device__ __forceinline__ void substep_multi_pass_seg(const StrandConsts& K, const SphereCache<M>& C,
-                                                       const SphereSet& S, int n, int iterations, V3 D0, V3 R,
-                                                       const XS& X, const VS& V) {
+template <bool PICK, bool FAST, typename XS, typename VS, int NF>
+__device__ __forceinline__ void substep_multi_pass_seg(const StrandConsts& K, const SphereFilter<NF>& F,
+                                                       const SphereSet& S, int n, int jmin, int iterations, V3 D0,
+                                                       V3 R, const XS& X, const VS& V) {
   for (int i = 1; i < n; ++i) {
     const float4 v = V.load(i);
     V.store(i, f4(disp(K, v), v.w));
@@ -563,7 +739,7 @@ __device__ __forceinline__ void substep_multi_pass_seg(const StrandConsts& K, co
       if (i >= 2) {
         const bool tip = i == n;
         V3 Dj = D_prev, sj = s_prev;
-        if (tests<NC>(C, w_prev)) push_seg<false, NC, FAST>(C, S, w_prev, Dj, sj, sn, tip);
+        if (i - 1 >= jmin && flagged(F, w_prev)) push_seg<PICK, FAST>(F, S, w_prev, Dj, sj, sn, tip);
         const V3 out = last ? vel_of(K, tip ? Dj : fmas(K.neg_damping, e, Dj)) : Dj;
         X.store(i - 1, f4(sj, rest_prev));
         V.store(i - 1, f4(out, vel_w<XS>(rest_prev)));
@@ -577,6 +753,26 @@ __device__ __forceinline__ void substep_multi_pass_seg(const StrandConsts& K, co
     V.fence();
   }
 }
+
+// The root over a frame: pinned, or linear from x0 to its target.
+struct RootPath {
+  V3 x0, target;
+  int substeps;
+  bool moving;
+  // Offset from the frame's start at the end of substep k: rel_k = alpha_k
+  // delta, delta itself at the last substep.
+  __device__ __forceinline__ V3 rel(int k) const {
+    if (!moving || k < 0) return v3(0.0f, 0.0f, 0.0f);
+    const V3 delta = sub(target, x0);
+    if (k + 1 == substeps) return delta;
+    return mul(__fdiv_rn(static_cast<float>(k + 1), static_cast<float>(substeps)), delta);
+  }
+  // Position at the end of substep k (rel: rel(k)).
+  __device__ __forceinline__ V3 at(int k, V3 rel) const {
+    if (!moving) return x0;
+    return k + 1 == substeps ? target : add(x0, rel);
+  }
+};
 
 // ---- the frame ------------------------------------------------------------
 
@@ -624,73 +820,67 @@ __device__ __forceinline__ V3 root_target(const FrameConst& fc, const GroomView&
   return target;
 }
 
-template <bool REF, int NC, bool SPLIT, bool CACHED, bool FAST, typename XS, typename VS, int M>
-__device__ __forceinline__ void substeps(const FrameConst& fc, const StrandConsts& K, const SphereCache<M>& C,
-                                         const SphereSet& S, int n, int jmin, V3 x0_start, V3 target, float rest0,
-                                         const XS& X, const VS& V) {
+template <int NC, typename XS, typename VS, int M>
+__device__ __forceinline__ void substeps_ref(const FrameConst& fc, const StrandConsts& K, const SphereCache<M>& C,
+                                             const SphereSet& S, int n, V3 x0_start, V3 target, float rest0,
+                                             const XS& X, const VS& V) {
   const bool moving = fc.root_mode != HS_ROOT_PINNED;
-  if constexpr (REF) {
-    const V3 root_delta = sub(target, x0_start);
-    V3 root = x0_start;  // root position at the start of the substep
-    for (int k = 0; k < fc.substeps; ++k) {
-      // Root (:184-193): kinematic, linear to its target, on it at the end.
-      V3 p0 = root;
-      if (moving) {
-        const float alpha = __fdiv_rn(static_cast<float>(k + 1), static_cast<float>(fc.substeps));
-        p0 = (k + 1 == fc.substeps) ? target : fmas(alpha, root_delta, x0_start);
-      }
-      const V3 v0 = sub(p0, root);  // :192
-      root = p0;
-      X.store(0, f4(p0, rest0));
-      V.store(0, f4(v0, vel_w<XS>(rest0)));
-      if (n >= 2) {
-        if (fc.iterations == 1) substep_single_pass_ref<NC>(K, C, S, n, p0, X, V);
-        else substep_multi_pass_ref<NC>(K, C, S, n, fc.iterations, p0, X, V);
-      }
-      V.fence();
+  const V3 root_delta = sub(target, x0_start);
+  V3 root = x0_start;  // root position at the start of the substep
+  for (int k = 0; k < fc.substeps; ++k) {
+    // Root (:184-193): kinematic, linear to its target, on it at the end.
+    V3 p0 = root;
+    if (moving) {
+      const float alpha = __fdiv_rn(static_cast<float>(k + 1), static_cast<float>(fc.substeps));
+      p0 = (k + 1 == fc.substeps) ? target : fmas(alpha, root_delta, x0_start);
     }
-  } else {
-    // Root offsets from the frame's start: rel_k = alpha_k delta (delta
-    // itself at the last substep), D_0 = rel_k - rel_{k-1}.
-    const V3 delta = sub(target, x0_start);
-    const V3 zero = v3(0.0f, 0.0f, 0.0f);
-    V3 rel_prev = zero, D0 = zero;
-    for (int k = 0; k < fc.substeps; ++k) {
-      V3 rel = zero, R = x0_start;
-      if (moving) {
-        const bool last = k + 1 == fc.substeps;
-        const float alpha = __fdiv_rn(static_cast<float>(k + 1), static_cast<float>(fc.substeps));
-        rel = last ? delta : mul(alpha, delta);
-        R = last ? target : add(x0_start, rel);
-      }
-      D0 = sub(rel, rel_prev);
-      rel_prev = rel;
-      if (n >= 2) {
-        if (fc.iterations == 1) substep_single_pass_seg<NC, SPLIT, CACHED, FAST>(K, C, S, n, jmin, D0, R, X, V);
-        else substep_multi_pass_seg<NC, FAST>(K, C, S, n, fc.iterations, D0, R, X, V);
-      }
-      V.fence();
+    const V3 v0 = sub(p0, root);  // :192
+    root = p0;
+    X.store(0, f4(p0, rest0));
+    V.store(0, f4(v0, vel_w<XS>(rest0)));
+    if (n >= 2) {
+      if (fc.iterations == 1) substep_single_pass_ref<NC>(K, C, S, n, p0, X, V);
+      else substep_multi_pass_ref<NC>(K, C, S, n, fc.iterations, p0, X, V);
     }
-    X.store(0, f4(zero, rest0));
-    V.store(0, f4(vel_of(K, D0), vel_w<XS>(rest0)));
     V.fence();
   }
+}
+
+// Substeps k0 .. substeps - 1, one at a time, then the root's slot.
+template <bool SPLIT, bool PICK, bool FAST, typename XS, typename VS, int NF>
+__device__ __forceinline__ void substeps_seg(const FrameConst& fc, const StrandConsts& K, const SphereFilter<NF>& F,
+                                             const SphereSet& S, int n, int jmin, int k0, V3 x0_start, V3 target,
+                                             float rest0, const XS& X, const VS& V) {
+  const RootPath path{x0_start, target, fc.substeps, fc.root_mode != HS_ROOT_PINNED};
+  V3 rel_prev = path.rel(k0 - 1);
+  for (int k = k0; k < fc.substeps; ++k) {
+    const V3 rel = path.rel(k), D0 = sub(rel, rel_prev), R = path.at(k, rel);
+    rel_prev = rel;
+    if (n >= 2) {
+      if (fc.iterations == 1) substep_single_pass_seg<SPLIT, PICK, FAST>(K, F, S, n, jmin, D0, R, X, V);
+      else substep_multi_pass_seg<PICK, FAST>(K, F, S, n, jmin, fc.iterations, D0, R, X, V);
+    }
+    V.fence();
+  }
+  const V3 D0 = sub(path.rel(fc.substeps - 1), path.rel(fc.substeps - 2));
+  X.store(0, f4(v3(0.0f, 0.0f, 0.0f), rest0));
+  V.store(0, f4(vel_of(K, D0), vel_w<XS>(rest0)));
+  V.fence();
 }
 
 // One frame of strand s. X: the position/segment slots (XShared4 or
 // XShared3, this thread's column of the block's shared [point][thread]
 // arrays); V: the velocity slots (VShared, or VTmem: whose loads and stores
 // are warp-collective, so every lane runs every pass, active or not).
-// M: sphere-cache width. With M = 8 a warp that reaches more than
-// kCachedSpheres spheres tests 8 cached ones instead of running the exact
-// push-out at every point; the others keep the 4-wide tests.
+// M (reference mode): sphere-cache width. With M = 8 a warp that reaches
+// more than kCachedSpheres spheres tests 8 cached ones instead of running
+// the exact push-out at every point; the others keep the 4-wide tests.
 // SPLIT: the DFTL pass shape (substep_single_pass_seg). One code shape per
-// kernel keeps the instruction cache warm: the batched kernels (4-wide
-// cache) run one loop; the plain step, whose 8-wide path splits, splits
-// both. CACHED: see push_seg (the plain step picks it for grooms with more
-// than 16 spheres).
-template <bool REF, typename XS, typename VS, int M = kCachedSpheres, bool SPLIT = (M > kCachedSpheres),
-          bool CACHED = false, bool FAST = false>
+// kernel keeps the instruction cache warm: the batched kernels run one
+// loop; the plain step splits it.
+// PICK: the push-out's form (push_seg).
+template <bool REF, typename XS, typename VS, int M = kCachedSpheres, bool SPLIT = false, bool PICK = false,
+          bool FAST = false>
 __device__ __forceinline__ void strand_frame_stream(const FrameConst& fc, const SphereSet& S, const GroomView& g,
                                                     uint32_t s, bool active, const XS& X, const VS& V) {
   const int n = static_cast<int>(g.npoints);
@@ -737,45 +927,51 @@ __device__ __forceinline__ void strand_frame_stream(const FrameConst& fc, const 
   const StrandConsts K = strand_consts(fc, g, s, active);
   const V3 target = root_target(fc, g, s, active, x0_start);
 
-  // Spheres this warp can touch during the frame (see hs_step.cuh), and
-  // the first point that can touch one: point j stays within R_j (its
+  // Spheres each strand can touch during the frame (see hs_step.cuh), and
+  // the warp's first point that can touch one: point j stays within R_j (its
   // links' lengths summed from the root) of the root, so it cannot reach
   // sphere k before R_j covers the distance from the root's path to k's
   // surface (same margins as near_spheres). A sphere reached only through
   // an overlap is entered by a point another sphere pushed first.
-  uint32_t reach = 0u;
-  int jmin = n;
-  if (S.n > 0) {
-    const V3 root_delta = sub(target, x0_start);
-    const V3 mid = v3(0.5f * (x0_start.x + target.x), 0.5f * (x0_start.y + target.y), 0.5f * (x0_start.z + target.z));
-    const float half_path = 0.5f * sqrtf(root_delta.x * root_delta.x + root_delta.y * root_delta.y +
-                                         root_delta.z * root_delta.z);
-    // Per lane: each thread caches the spheres its own strand can reach, so
-    // a warp whose strands lie far apart (a mesh's vertex order, or any
-    // order) tests no more than spatially coherent ones do.
-    reach = active ? overlap_closure(S, near_spheres(S, mid, R + half_path)) : 0u;
-    const float thr = reach_threshold(S, mid, R + half_path, half_path);
-    float Rj = 0.0f;
-    int jl = n;
-    for (int i = 1; i < n; ++i) {  // the same sum as R, point by point
-      const float rest = with_rest<XS>(X.load(i), V.load(i)).w;
-      Rj += fabsf(fc.length_scale * rest);
-      if (jl == n && Rj >= thr) jl = i;
+  if constexpr (REF) {
+    uint32_t reach = 0u;
+    if (S.n > 0) {
+      const V3 root_delta = sub(target, x0_start);
+      const V3 mid = v3(0.5f * (x0_start.x + target.x), 0.5f * (x0_start.y + target.y), 0.5f * (x0_start.z + target.z));
+      const float half_path = 0.5f * sqrtf(root_delta.x * root_delta.x + root_delta.y * root_delta.y +
+                                           root_delta.z * root_delta.z);
+      reach = active ? overlap_closure(S, near_spheres(S, mid, R + half_path)) : 0u;
     }
-    jmin = __reduce_min_sync(0xffffffffu, active ? jl : n);
+    const SphereCache<M> C = cache_spheres<M>(S, reach);
+    // All tested slots are tested whether filled or not (empty ones never
+    // hit). The width is chosen per warp.
+    const int warp_cached = __reduce_max_sync(0xffffffffu, C.ncached);
+    if (M > kCachedSpheres && warp_cached > kCachedSpheres)
+      substeps_ref<M>(fc, K, C, S, n, x0_start, target, rest0, X, V);
+    else
+      substeps_ref<kCachedSpheres>(fc, K, C, S, n, x0_start, target, rest0, X, V);
+  } else {
+    uint32_t reach = 0u;
+    int jmin = n;
+    float far = 0.0f;
+    if (S.n > 0) {
+      const StrandBall ball(x0_start, target, R);
+      const SphereReach q = sphere_reach(S, ball);
+      reach = active ? overlap_closure(S, q.near) : 0u;
+      far = ball.far();
+      if (__any_sync(0xffffffffu, reach)) {
+        float Rj = 0.0f;
+        int jl = n;
+        for (int i = 1; i < n; ++i) {  // the same sum as R, point by point
+          Rj += fabsf(fc.length_scale * rest_of(X, V, i));
+          if (jl == n && Rj >= q.threshold) jl = i;
+        }
+        jmin = __reduce_min_sync(0xffffffffu, active ? jl : n);
+      }
+    }
+    const SphereFilter<8> F = filter_spheres<8>(S, reach, far);
+    substeps_seg<SPLIT, PICK, FAST>(fc, K, F, S, n, jmin, 0, x0_start, target, rest0, X, V);
   }
-  const SphereCache<M> C = cache_spheres<M>(S, reach);
-  // One code path per cache width: all tested slots are tested whether
-  // filled or not (empty ones never hit). A second path without sphere
-  // tests saved their cost for warps that reach no sphere, but warps on
-  // different paths at once thrashed the instruction cache of the batched
-  // kernels (measured: one path is 13-16 % faster on the batched workload
-  // and no slower on a single groom). The width is chosen per warp.
-  const int warp_cached = __reduce_max_sync(0xffffffffu, C.ncached);
-  if (M > kCachedSpheres && warp_cached > kCachedSpheres)
-    substeps<REF, M, SPLIT, CACHED, FAST>(fc, K, C, S, n, jmin, x0_start, target, rest0, X, V);
-  else
-    substeps<REF, kCachedSpheres, SPLIT, CACHED, FAST>(fc, K, C, S, n, jmin, x0_start, target, rest0, X, V);
 
   // Store: reference mode holds positions; DFTL mode rebuilds them from the
   // final root and the segments.
@@ -841,14 +1037,13 @@ __device__ __forceinline__ void strand_frame_regs_dftl(const FrameConst& fc, con
   const V3 target = root_target(fc, g, s, active, x0_start);
   const bool moving = fc.root_mode != HS_ROOT_PINNED;
   uint32_t reach = 0u;
+  float far = 0.0f;
   if (S.n > 0) {
-    const V3 root_delta = sub(target, x0_start);
-    const V3 mid = v3(0.5f * (x0_start.x + target.x), 0.5f * (x0_start.y + target.y), 0.5f * (x0_start.z + target.z));
-    const float half_path = 0.5f * sqrtf(root_delta.x * root_delta.x + root_delta.y * root_delta.y +
-                                         root_delta.z * root_delta.z);
-    reach = active ? overlap_closure(S, near_spheres(S, mid, R + half_path)) : 0u;  // per lane
+    const StrandBall ball(x0_start, target, R);
+    reach = active ? overlap_closure(S, near_spheres(S, ball.mid, ball.radius)) : 0u;  // per lane
+    far = ball.far();
   }
-  const SphereCache<kCachedSpheres> C = cache_spheres<kCachedSpheres>(S, reach);
+  const SphereFilter<4> F = filter_spheres<4>(S, reach, far);
 
   const V3 delta = sub(target, x0_start);
   V3 rel_prev = zero, D0 = zero;
@@ -889,8 +1084,7 @@ __device__ __forceinline__ void strand_frame_regs_dftl(const FrameConst& fc, con
           if (i >= 2) {
             const bool tip = i == n;
             V3 Dj = D_prev, sj = s_prev;
-            if (tests<kCachedSpheres>(C, w_prev))
-              push_seg<false, kCachedSpheres, FAST>(C, S, w_prev, Dj, sj, sn, tip);
+            if (flagged(F, w_prev)) push_seg<false, FAST>(F, S, w_prev, Dj, sj, sn, tip);
             const V3 out = last_it ? vel_of(K, tip ? Dj : fmas(K.neg_damping, e, Dj)) : Dj;
             Sg[i - 1] = sj;
             vs.set(i - 1, f4(out, rest_prev));

@@ -81,6 +81,15 @@ struct VTmem {
   __device__ __forceinline__ float4 load(int i) const {
     return tmem::load4(lane_addr + 4u * static_cast<uint32_t>(i));
   }
+  __device__ __forceinline__ float load_w(int i) const {  // the fourth column alone
+    uint32_t r;
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];\n\t"
+                 "tcgen05.wait::ld.sync.aligned;"
+                 : "=r"(r)
+                 : "r"(lane_addr + 4u * static_cast<uint32_t>(i) + 3u)
+                 : "memory");
+    return __uint_as_float(r);
+  }
   __device__ __forceinline__ void store(int i, float4 v) const {
     tmem::store4(lane_addr + 4u * static_cast<uint32_t>(i), v);
   }
