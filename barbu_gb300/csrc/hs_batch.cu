@@ -152,9 +152,11 @@ __global__ void __maxnreg__(128)
 // memory holds the table entries and the positions, 12 bytes a point.
 // WARPS (4 or 8) is compile-time, so the shared-memory strides are
 // immediates; resident blocks are bounded by TMEM and shared memory at 16
-// warps per SM, so registers are held to 128 a thread.
-template <bool REF, int WARPS, bool FAST>
-__global__ void __launch_bounds__(WARPS * 32, 16 / WARPS)
+// warps per SM (8 for more than 32 points), and registers with them. P:
+// pairs of substeps at once (WavePass): none, or 1 for a bucket of less than
+// a wave of warps, 2 for more than 32 points.
+template <bool REF, int WARPS, bool FAST, int P>
+__global__ void __launch_bounds__(WARPS * 32, (P == 2 ? 8 : 16) / WARPS)
     k_step_batch_stream_tmem(const BucketHeader* __restrict__ hdr, const BucketDir* __restrict__ dirs,
                              const BatchGroomDev* __restrict__ table, uint32_t* __restrict__ counters, int bucket,
                              int cap) {
@@ -191,8 +193,8 @@ __global__ void __launch_bounds__(WARPS * 32, 16 / WARPS)
     }
     const uint32_t s = strand0 + lane;
     const SphereSet S{e.fc.spheres, e.fc.r2, e.fc.adj, e.fc.nspheres};
-    strand_frame_stream<REF, XShared3, VTmem, kCachedSpheres, false, false, FAST>(e.fc, S, e.view, s,
-                                                                                 s < e.view.nstrands, X, V);
+    strand_frame_stream<REF, XShared3, VTmem, kCachedSpheres, false, false, FAST, P, P == 1 ? 4 : 8>(
+        e.fc, S, e.view, s, s < e.view.nstrands, X, V);
   }
   tmem::fence_before_sync();
   __syncthreads();
@@ -242,8 +244,16 @@ __global__ void __launch_bounds__(K * 32, 16 / K)
   }
 }
 
+template <bool REF, bool FAST, int P>
+const void* tmem_kernel(int warps) {
+  if (warps == 4) return reinterpret_cast<const void*>(&k_step_batch_stream_tmem<REF, 4, FAST, P>);
+  if (warps == 8) return reinterpret_cast<const void*>(&k_step_batch_stream_tmem<REF, 8, FAST, P>);
+  return nullptr;
+}
+
+// pairs: pairs of substeps at once (tensor-memory DFTL kernels).
 template <bool REF, bool FAST>
-const void* any_cap_kernel(int variant, int warps) {
+const void* any_cap_kernel(int variant, int warps, int pairs) {
   if (is_lanes(variant)) {
     if (REF) return nullptr;
     if (warps == 2) return reinterpret_cast<const void*>(&k_step_batch_lanes<2, FAST>);
@@ -253,9 +263,11 @@ const void* any_cap_kernel(int variant, int warps) {
     return nullptr;
   }
   if (is_tmem(variant)) {
-    if (warps == 4) return reinterpret_cast<const void*>(&k_step_batch_stream_tmem<REF, 4, FAST>);
-    if (warps == 8) return reinterpret_cast<const void*>(&k_step_batch_stream_tmem<REF, 8, FAST>);
-    return nullptr;
+    if constexpr (!REF) {
+      if (pairs == 1) return tmem_kernel<REF, FAST, 1>(warps);
+      if (pairs == 2) return tmem_kernel<REF, FAST, 2>(warps);
+    }
+    return tmem_kernel<REF, FAST, 0>(warps);
   }
   if (is_stream(variant)) return reinterpret_cast<const void*>(&k_step_batch_stream<REF, FAST>);
   return nullptr;
@@ -264,35 +276,35 @@ const void* any_cap_kernel(int variant, int warps) {
 // Register variants exist for short strands only (up to 8 points): longer
 // register-resident strands spill.
 template <int CAP, bool REF, bool FAST>
-const void* batch_kernel(int variant, int warps) {
-  if (any_capacity(variant)) return any_cap_kernel<REF, FAST>(variant, warps);
+const void* batch_kernel(int variant, int warps, int pairs) {
+  if (any_capacity(variant)) return any_cap_kernel<REF, FAST>(variant, warps, pairs);
   if (variant == kVariantRegsVsmem) return reinterpret_cast<const void*>(&k_step_batch<CAP, REF, true, FAST>);
   if (variant == kVariantRegs) return reinterpret_cast<const void*>(&k_step_batch<CAP, REF, false, FAST>);
   return nullptr;
 }
 
 template <int CAP>
-const void* class_kernel(int cls, int variant, int warps) {
+const void* class_kernel(int cls, int variant, int warps, int pairs) {
   if constexpr (CAP <= 8) {
-    if (cls == kClassRef) return batch_kernel<CAP, true, false>(variant, warps);
-    if (cls == kClassFast) return batch_kernel<CAP, false, true>(variant, warps);
-    return batch_kernel<CAP, false, false>(variant, warps);
+    if (cls == kClassRef) return batch_kernel<CAP, true, false>(variant, warps, pairs);
+    if (cls == kClassFast) return batch_kernel<CAP, false, true>(variant, warps, pairs);
+    return batch_kernel<CAP, false, false>(variant, warps, pairs);
   } else {
-    if (cls == kClassRef) return any_cap_kernel<true, false>(variant, warps);
-    if (cls == kClassFast) return any_cap_kernel<false, true>(variant, warps);
-    return any_cap_kernel<false, false>(variant, warps);
+    if (cls == kClassRef) return any_cap_kernel<true, false>(variant, warps, pairs);
+    if (cls == kClassFast) return any_cap_kernel<false, true>(variant, warps, pairs);
+    return any_cap_kernel<false, false>(variant, warps, pairs);
   }
 }
 
 // The kernel of a bucket shape (null where the shape is not built).
-const void* kernel_for(int cap, int cls, int variant, int warps) {
+const void* kernel_for(int cap, int cls, int variant, int warps, int pairs) {
   switch (cap) {
-    case 4: return class_kernel<4>(cls, variant, warps);
-    case 8: return class_kernel<8>(cls, variant, warps);
+    case 4: return class_kernel<4>(cls, variant, warps, pairs);
+    case 8: return class_kernel<8>(cls, variant, warps, pairs);
     case 16:
     case 24:
     case 32:
-    case 64: return class_kernel<64>(cls, variant, warps);
+    case 64: return class_kernel<64>(cls, variant, warps, pairs);
     default: return nullptr;
   }
 }
@@ -351,7 +363,7 @@ void fill_args(const BatchState& B, int b, LaunchArgs* a) {
 
 cudaKernelNodeParams node_params(const Bucket& bk, LaunchArgs* a) {
   cudaKernelNodeParams p{};
-  p.func = const_cast<void*>(kernel_for(bk.cap, bk.cls, bk.variant, bk.warps_per_block));
+  p.func = const_cast<void*>(kernel_for(bk.cap, bk.cls, bk.variant, bk.warps_per_block, bk.pairs));
   p.gridDim = dim3(bk.grid);
   p.blockDim = dim3(bk.warps_per_block * kWarp);
   p.sharedMemBytes = static_cast<unsigned>(smem_bytes(bk.cap, bk.warps_per_block, bk.variant));
@@ -362,8 +374,22 @@ cudaKernelNodeParams node_params(const Bucket& bk, LaunchArgs* a) {
 
 }  // namespace
 
-int batch_occupancy(int cap, int cls, int variant, int warps_per_block) {
-  const void* fn = kernel_for(cap, cls, variant, warps_per_block);
+// Pairs of substeps a bucket of `ntiles` 32-strand tiles runs at once: two
+// for more than 32 points (8 warps an SM), one where its tiles are no more
+// than the 16 warps an SM holds (48 grooms of 256 - 4,096 strands, 2,054
+// tiles on 2,432 warps: 48 - 58 -> 40 - 42 us a frame; 4,155 tiles of such
+// grooms: 63 -> 72 us, where the GPU is busy with other work too), else
+// none. (The occupancy query answers one block an SM for kernels that
+// allocate tensor memory, so it does not say how many warps there are.)
+static int substep_pairs(int cap, int cls, int variant, uint32_t ntiles) {
+  if (!is_tmem(variant) || cls == kClassRef) return 0;
+  if (cap > 32) return 2;
+  const int sms = device_attribute(cudaDevAttrMultiProcessorCount, 152);
+  return ntiles <= 16u * static_cast<uint32_t>(sms) ? 1 : 0;
+}
+
+int batch_occupancy(int cap, int cls, int variant, int warps_per_block, int pairs) {
+  const void* fn = kernel_for(cap, cls, variant, warps_per_block, pairs);
   if (!fn) return 0;
   const size_t smem = smem_bytes(cap, warps_per_block, variant);
   // Buckets of different capacities share the streaming kernel: opt every
@@ -565,7 +591,8 @@ static void regroup(hs_ctx* ctx, BatchState& B, hs_groom* const* grooms, uint32_
     if (!shape_fits(bk, tc)) tc = default_choice(bk.cap);
     bk.variant = tc.variant;
     bk.warps_per_block = tc.warps_per_block;
-    const int occ = std::max(1, batch_occupancy(bk.cap, bk.cls, bk.variant, bk.warps_per_block));
+    bk.pairs = substep_pairs(bk.cap, bk.cls, bk.variant, tiles);
+    const int occ = std::max(1, batch_occupancy(bk.cap, bk.cls, bk.variant, bk.warps_per_block, bk.pairs));
     bk.grid = static_cast<uint32_t>(sms * occ * tc.waves);
     // Bucket b of the launch reads header and counter slot b.
     B.headers[B.buckets.size()] = h;
@@ -596,6 +623,7 @@ static std::vector<int64_t> shape_of(const BatchState& B) {
     s.push_back(bk.cls);
     s.push_back(bk.variant);
     s.push_back(bk.warps_per_block);
+    s.push_back(bk.pairs);
     s.push_back(bk.grid);
   }
   return s;
@@ -742,12 +770,13 @@ static hs_status autotune(hs_ctx* ctx, hs_groom* const* grooms, uint32_t n, floa
       for (int wpb : {1, 2, 4, 8, 16}) {
         if (!shape_fits(bk, TuneChoice{wpb, 1, variant})) continue;
         if (wpb == 16 && !is_lanes(variant)) continue;
-        const int occ = batch_occupancy(bk.cap, bk.cls, variant, wpb);
+        Bucket trial = bk;
+        trial.variant = variant;
+        trial.warps_per_block = wpb;
+        trial.pairs = substep_pairs(bk.cap, bk.cls, variant, bk.ntiles);
+        const int occ = batch_occupancy(bk.cap, bk.cls, variant, wpb, trial.pairs);
         if (occ <= 0) continue;
         for (int waves : {1, 2, 4}) {
-          Bucket trial = bk;
-          trial.variant = variant;
-          trial.warps_per_block = wpb;
           trial.grid = static_cast<uint32_t>(sms * occ * waves);
           LaunchArgs a;
           fill_args(B, static_cast<int>(b), &a);
@@ -844,8 +873,9 @@ HS_API hs_status hs_tune_override(hs_ctx* ctx, uint32_t points, uint32_t mode, u
   if (is_lanes(static_cast<int>(variant)) && mode != HS_MODE_DFTL)
     return fail(HS_ERR_UNSUPPORTED, "hs_tune_override: lane groups run DFTL mode only");
   if (waves != 1 && waves != 2 && waves != 4) return fail(HS_ERR_INVALID_ARG, "hs_tune_override: waves must be 1, 2 or 4");
-  if (batch_occupancy(cap, mode == HS_MODE_REFERENCE ? kClassRef : kClassExact, static_cast<int>(variant),
-                      static_cast<int>(warps_per_block)) <= 0)
+  const int cls = mode == HS_MODE_REFERENCE ? kClassRef : kClassExact;
+  if (batch_occupancy(cap, cls, static_cast<int>(variant), static_cast<int>(warps_per_block),
+                      substep_pairs(cap, cls, static_cast<int>(variant), 1)) <= 0)
     return fail(HS_ERR_UNSUPPORTED, "hs_tune_override: that shape does not fit on an SM");
   if (!ctx->tune) ctx->tune = new TuneCache();
   ctx->tune->pinned[std::make_pair(cap, mode == HS_MODE_REFERENCE)] =
@@ -1002,7 +1032,7 @@ hs_status noalloc_setup(int device, NoAllocDevice* out) {
     if (e != cudaSuccess) return cuda_fail(e, "hs_update_many_noalloc: SM count");
     for (int cap : kNoAllocCaps) {
       for (int cls = 0; cls < kClasses; ++cls) {
-        const int occ = batch_occupancy(cap, cls, kVariantStream, 1);
+        const int occ = batch_occupancy(cap, cls, kVariantStream, 1, 0);
         if (occ <= 0) return fail(HS_ERR_UNSUPPORTED, "hs_update_many_noalloc: %d-point step does not fit", cap);
         d.occupancy[bucket_slot(cap, cls)] = occ;
       }
@@ -1080,7 +1110,7 @@ hs_status noalloc_update(hs_ctx* ctx, hs_groom* const* grooms, uint32_t n, float
     int cap_arg = cap;
     void* args[6] = {&hdr, &dirs, &table, &counters, &bucket, &cap_arg};
     const dim3 grid(static_cast<unsigned>(dev->sms * dev->occupancy[b]));
-    e = cudaLaunchKernel(kernel_for(cap, cls, kVariantStream, 1), grid, dim3(kWarp), args,
+    e = cudaLaunchKernel(kernel_for(cap, cls, kVariantStream, 1, 0), grid, dim3(kWarp), args,
                          smem_bytes(cap, 1, kVariantStream), stream);
     ++launches;
   }

@@ -75,6 +75,7 @@ struct Bucket {
   int cls = kClassExact;  // step class
   int variant = kVariantRegs;
   int warps_per_block = 4;
+  int pairs = 0;  // pairs of substeps the kernel runs at once (substep_pairs)
   uint32_t grid = 1;
   uint32_t ntiles = 0;
   int lanes_k = 0;  // smallest lane group every groom of the bucket fits (0: none, lane_group)
@@ -127,7 +128,8 @@ struct TuneCache {
 TuneKey tune_key(int cap, int cls, uint32_t ntiles);
 TuneChoice tuned_choice(hs_ctx* ctx, int cap, int cls, uint32_t ntiles);
 TuneChoice default_choice(int cap);  // the untuned shape of a capacity
-int batch_occupancy(int cap, int cls, int variant, int warps_per_block);
+// pairs: pairs of substeps at once (Bucket::pairs).
+int batch_occupancy(int cap, int cls, int variant, int warps_per_block, int pairs);
 hs_status batch_update(hs_ctx* ctx, hs_groom* const* grooms, uint32_t n, float dt);
 
 }  // namespace hs

@@ -93,6 +93,81 @@ __device__ __forceinline__ float rsqrt_fast(float x) {
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(fmaxf(x, 1.17549435e-38f)));
   return y;
 }
+// Two floats (or two vectors, component by component) in 64-bit registers,
+// for the same operation of two substeps as one two-wide instruction a
+// component: `lo` of one, `hi` of the other. They stay in that form from
+// operation to operation (scalars that are packed anew for each would cost
+// a register move each). Each half is rounded as the scalar .rn instruction
+// rounds it.
+struct F2 {
+  uint64_t v;
+};
+__device__ __forceinline__ F2 f2(float a, float b) { return F2{pair(a, b)}; }
+__device__ __forceinline__ float lo(F2 a) {
+  float x;
+  asm("{\n\t.reg .f32 t;\n\tmov.b64 {%0, t}, %1;\n\t}" : "=f"(x) : "l"(a.v));
+  return x;
+}
+__device__ __forceinline__ float hi(F2 a) {
+  float y;
+  asm("{\n\t.reg .f32 t;\n\tmov.b64 {t, %0}, %1;\n\t}" : "=f"(y) : "l"(a.v));
+  return y;
+}
+struct V3x2 {
+  F2 x, y, z;
+};
+__device__ __forceinline__ F2 add2(F2 a, F2 b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a.v), "l"(b.v));
+  return F2{r};
+}
+__device__ __forceinline__ F2 sub2(F2 a, F2 b) {
+  uint64_t r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a.v), "l"(b.v));
+  return F2{r};
+}
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return F2{r};
+}
+// Only where the product feeds no two-wide addition or subtraction (ptxas
+// would fuse the two, see above).
+__device__ __forceinline__ F2 mul2(F2 a, F2 b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a.v), "l"(b.v));
+  return F2{r};
+}
+// a * b rounded once where the product does feed one: a fused multiply-add
+// with the addend -0 (x + -0 is x for every x, signed zeros included), which
+// leaves no product to fuse. `neg0` is negative_zero(), a pair of -0 that
+// the compiler cannot know.
+__device__ __forceinline__ F2 mul2_kept(F2 a, F2 b, F2 neg0) { return fma2(a, b, neg0); }
+__device__ __forceinline__ F2 negative_zero() {
+  const float z = __uint_as_float(0x80000000u | threadIdx.z);  // one-dimensional blocks: threadIdx.z is 0
+  return f2(z, z);
+}
+__device__ __forceinline__ V3x2 add2(V3x2 a, V3x2 b) { return V3x2{add2(a.x, b.x), add2(a.y, b.y), add2(a.z, b.z)}; }
+__device__ __forceinline__ V3x2 sub2(V3x2 a, V3x2 b) { return V3x2{sub2(a.x, b.x), sub2(a.y, b.y), sub2(a.z, b.z)}; }
+__device__ __forceinline__ V3x2 mul2_kept(F2 s, V3x2 a, F2 neg0) {
+  return V3x2{mul2_kept(s, a.x, neg0), mul2_kept(s, a.y, neg0), mul2_kept(s, a.z, neg0)};
+}
+__device__ __forceinline__ F2 dot2(V3x2 a, V3x2 b) { return fma2(a.z, b.z, fma2(a.y, b.y, mul2(a.x, b.x))); }
+__device__ __forceinline__ V3 lo(V3x2 a) { return V3{lo(a.x), lo(a.y), lo(a.z)}; }
+__device__ __forceinline__ V3 hi(V3x2 a) { return V3{hi(a.x), hi(a.y), hi(a.z)}; }
+__device__ __forceinline__ V3x2 v3x2(V3 a, V3 b) { return V3x2{f2(a.x, b.x), f2(a.y, b.y), f2(a.z, b.z)}; }
+// inversesqrt of both halves, operation for operation; rsqrt_fast of both.
+__device__ __forceinline__ F2 inversesqrt2(F2 x) {
+  const float xa = lo(x), xb = hi(x);
+  F2 y = f2(__uint_as_float(0x5f3759dfu - (__float_as_uint(xa) >> 1)),
+            __uint_as_float(0x5f3759dfu - (__float_as_uint(xb) >> 1)));
+  const F2 nhx = mul2(f2(-0.5f, -0.5f), x);
+  y = mul2(y, fma2(nhx, mul2(y, y), f2(1.5f, 1.5f)));
+  y = mul2(y, fma2(nhx, mul2(y, y), f2(1.5f, 1.5f)));
+  const F2 nxy = mul2(f2(-xa, -xb), y);
+  return fma2(mul2(f2(0.5f, 0.5f), y), fma2(nxy, y, f2(1.0f, 1.0f)), y);
+}
+__device__ __forceinline__ F2 rsqrt_fast2(F2 x) { return f2(rsqrt_fast(lo(x)), rsqrt_fast(hi(x))); }
 __device__ __forceinline__ V3 reflect(V3 i, V3 n) { return sub(i, mul(__fmul_rn(2.0f, dot(n, i)), n)); }
 
 // Seeded counter hash (lowbias32, C. Wellons), standing in for the

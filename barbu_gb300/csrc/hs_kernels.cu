@@ -127,9 +127,11 @@ __global__ void __launch_bounds__(kStreamBlock) k_step_stream(GroomView g, Frame
 // TMEM velocity slots).
 constexpr int kTmemBlock = 128;
 
-// MANY: the push-out's form for grooms among many spheres (push_seg).
-template <bool REF, bool MANY, bool FAST>
-__global__ void __launch_bounds__(kTmemBlock) k_step_stream_tmem(GroomView g, FrameConst fc) {
+// MANY: the push-out's form for grooms among many spheres (push_seg). LONG:
+// more than 32 points, where tensor memory holds two blocks an SM: four
+// substeps at once (WavePass).
+template <bool REF, bool MANY, bool LONG, bool FAST>
+__global__ void __launch_bounds__(kTmemBlock, LONG ? 2 : 4) k_step_stream_tmem(GroomView g, FrameConst fc) {
   extern __shared__ float4 s_pos[];  // positions, compact: float2 (x, y) then float z, each [npoints][kTmemBlock]
   __shared__ float4 s_c[HS_MAX_SPHERES];
   __shared__ float s_r2[HS_MAX_SPHERES];
@@ -153,7 +155,7 @@ __global__ void __launch_bounds__(kTmemBlock) k_step_stream_tmem(GroomView g, Fr
   float2* xy = reinterpret_cast<float2*>(s_pos);
   float* z = reinterpret_cast<float*>(xy + g.npoints * kTmemBlock);
   const XShared3 X{xy + threadIdx.x, z + threadIdx.x, kTmemBlock};
-  strand_frame_stream<REF, XShared3, VTmem, 8, true, MANY, FAST>(fc, S, g, s, s < g.nstrands, X, V);
+  strand_frame_stream<REF, XShared3, VTmem, 8, true, MANY, FAST, LONG ? 2 : 0>(fc, S, g, s, s < g.nstrands, X, V);
   tmem::fence_before_sync();
   __syncthreads();
   tmem::fence_after_sync();
@@ -178,9 +180,10 @@ size_t tmem_step_smem(uint32_t npoints) {
 constexpr int kFewSpheres = 8;
 
 using TmemStep = void (*)(GroomView, FrameConst);
-TmemStep dftl_step_tmem(bool many, bool fast) {
-  if (many) return fast ? k_step_stream_tmem<false, true, true> : k_step_stream_tmem<false, true, false>;
-  return fast ? k_step_stream_tmem<false, false, true> : k_step_stream_tmem<false, false, false>;
+TmemStep dftl_step_tmem(bool many, bool is_long, bool fast) {
+  if (is_long) return fast ? k_step_stream_tmem<false, false, true, true> : k_step_stream_tmem<false, false, true, false>;
+  if (many) return fast ? k_step_stream_tmem<false, true, false, true> : k_step_stream_tmem<false, true, false, false>;
+  return fast ? k_step_stream_tmem<false, false, false, true> : k_step_stream_tmem<false, false, false, false>;
 }
 
 cudaError_t launch_step_stream_tmem(const GroomView& g, const FrameConst& fc, cudaStream_t st) {
@@ -191,12 +194,15 @@ cudaError_t launch_step_stream_tmem(const GroomView& g, const FrameConst& fc, cu
     const int bytes = 200 * 1024;
     for (const bool fast : {false, true})
       for (const bool many : {false, true})
-        cudaFuncSetAttribute(dftl_step_tmem(many, fast), cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    cudaFuncSetAttribute(k_step_stream_tmem<true, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        for (const bool is_long : {false, true})
+          cudaFuncSetAttribute(dftl_step_tmem(many, is_long, fast), cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    cudaFuncSetAttribute(k_step_stream_tmem<true, false, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         bytes);
   });
   if (fc.mode == HS_MODE_REFERENCE)
-    return launch_overlapped(k_step_stream_tmem<true, false, false>, grid, kTmemBlock, smem, st, g, fc);
-  return launch_overlapped(dftl_step_tmem(fc.nspheres > kFewSpheres, fast_frame(fc)), grid, kTmemBlock, smem, st, g, fc);
+    return launch_overlapped(k_step_stream_tmem<true, false, false, false>, grid, kTmemBlock, smem, st, g, fc);
+  return launch_overlapped(dftl_step_tmem(fc.nspheres > kFewSpheres, g.npoints > 32, fast_frame(fc)), grid, kTmemBlock,
+                           smem, st, g, fc);
 }
 
 // Lane groups (hs_lanes.cuh): a block of K warps per 32-strand tile, the

@@ -774,6 +774,298 @@ struct RootPath {
   }
 };
 
+// ---- several substeps at once --------------------------------------------
+
+// Two-wide form of a strand's sphere filter.
+template <int NF>
+struct SphereFilter2 {
+  F2 cx[NF], cy[NF], cz[NF], k[NF];
+  uint32_t reach;
+  bool many, most;
+  explicit __device__ __forceinline__ SphereFilter2(const SphereFilter<NF>& F)
+      : reach(F.reach), many(F.many), most(F.most) {
+#pragma unroll
+    for (int q = 0; q < NF; ++q) {
+      cx[q] = f2(F.cx[q], F.cx[q]);
+      cy[q] = f2(F.cy[q], F.cy[q]);
+      cz[q] = f2(F.cz[q], F.cz[q]);
+      k[q] = f2(F.k[q], F.k[q]);
+    }
+  }
+  __device__ __forceinline__ F2 value(int q, V3x2 w) const {
+    return fma2(cx[q], w.x, fma2(cy[q], w.y, fma2(cz[q], w.z, k[q])));
+  }
+  // Whether one of the two points may be inside a sphere.
+  __device__ __forceinline__ bool flagged(V3x2 w) const {
+    const F2 w2 = dot2(w, w);
+    F2 v = value(0, w), u = value(1, w);
+    float ma = fminf(lo(v), lo(u)), mb = fminf(hi(v), hi(u));
+    if (many) {
+#pragma unroll
+      for (int q = 2; q < 4; ++q) {
+        v = value(q, w);
+        ma = fminf(ma, lo(v));
+        mb = fminf(mb, hi(v));
+      }
+      if (NF > 4 && most) {
+#pragma unroll
+        for (int q = 4; q < NF; ++q) {
+          v = value(q, w);
+          ma = fminf(ma, lo(v));
+          mb = fminf(mb, hi(v));
+        }
+      }
+    }
+    return ma <= -lo(w2) || mb <= -hi(w2);
+  }
+};
+
+// Points a strand needs for W substeps at once: the first stage's loads of a
+// sweep stay behind the last one's stores of the one before.
+template <int W>
+constexpr int kWaveMinPoints = 4 * W;
+
+// Two stages of the pipeline as the halves of pairs (the earlier substep in
+// the low halves): the point to link next (its segment plus displacement a,
+// displacement d, rest length) and the one linked last (displacement D,
+// chain position w, segment s, rest length).
+struct WaveStages {
+  V3x2 a, d, D, w, s;
+  float next_a, next_b, last_a, last_b;
+};
+struct WaveLinked {
+  V3x2 s, e, D, w;
+};
+
+// Substeps k0 + W r .. k0 + W r + W - 1, r = 0 .. sweeps - 1 (W = 2 P), each
+// W of them one sweep over the points, as the stages of a pipeline: stage k
+// takes the points stage k - 1 has finished from registers, so the slots are
+// read and written once every W substeps, and two stages are the halves of
+// two-wide FP32 instructions (F2). The arithmetic of a point and substep is
+// SegPass::step's, operation for operation.
+//
+// It is for strands whose warps wait on their chain links: where a warp or
+// two a scheduler run (33 to 64 points, tensor memory's limit), or less
+// than a wave of warps. The steps between sweeps and the moves between the
+// halves cost what the shared loads and stores save in instructions, so
+// that with 16 busy warps an SM the single pass is faster (64 grooms: 1,150
+// against 880 us).
+//
+// Step i of a sweep links point i - 2k
+// in stage k and finishes point i - 2k - 1. The sweeps follow each other
+// without a gap: while the last stages end a sweep, the first ones are at
+// the first points of the next. The 2 W + 1 steps where a stage starts or
+// ends run in `edge` (t = i - (n - 1), which are i = 0, 1, .. of the next
+// sweep), the others in `step`. Slot 0 holds the root meanwhile (X: where it
+// starts, V: its target).
+template <int P, bool FAST, typename XS, typename VS, int NF>
+struct WavePass {
+  static constexpr int W = 2 * P;
+  const StrandConsts& K;
+  const FrameConst& fc;
+  const SphereFilter2<NF>& F;
+  const SphereSet& S;
+  const XS& X;
+  const VS& V;
+  int n, jmin, k0;
+  F2 neg0;
+  WaveStages st[P];
+
+  __device__ __forceinline__ WaveLinked link(const WaveStages& q) const {
+    WaveLinked l;
+    const V3x2 d = sub2(q.a, q.D);
+    const F2 d2 = dot2(d, d);
+    const F2 rs = FAST ? rsqrt_fast2(d2) : inversesqrt2(d2);
+    const F2 sc = f2(__fmul_rn(__fmul_rn(K.lscale, q.next_a), lo(rs)), __fmul_rn(__fmul_rn(K.lscale, q.next_b), hi(rs)));
+    l.s = mul2_kept(sc, d, neg0);
+    l.e = sub2(l.s, d);
+    l.D = add2(q.d, l.e);
+    l.w = add2(q.w, l.s);
+    return l;
+  }
+  // The in-order push-out (push_seg) of both stages' points linked last.
+  // `ta`, `tb`: whether the stage's point is tested.
+  __device__ __forceinline__ void push(bool ta, bool tb, WaveStages& st, V3x2& s_next) const {
+    V3x2 p = st.w;
+    bool pa = false, pb = false;
+    for (uint32_t m = F.reach; m; m &= m - 1u) {
+      const int k = __ffs(m) - 1;
+      const float4 c = S.c[k];
+      const float r2 = S.r2[k];
+      const V3x2 cc = V3x2{f2(c.x, c.x), f2(c.y, c.y), f2(c.z, c.z)};
+      const V3x2 d = sub2(p, cc);
+      const F2 dp = dot2(d, d);
+      const bool ha = ta && lo(dp) < r2, hb = tb && hi(dp) < r2;
+      if (ha || hb) {
+        const V3x2 u = mul2_kept(FAST ? rsqrt_fast2(dp) : inversesqrt2(dp), d, neg0);
+        const bool oa = lo(dp) > 0.0f, ob = hi(dp) > 0.0f;  // not at the centre
+        const V3x2 nn = V3x2{f2(oa ? lo(u.x) : 0.0f, ob ? hi(u.x) : 0.0f), f2(oa ? lo(u.y) : 1.0f, ob ? hi(u.y) : 1.0f),
+                             f2(oa ? lo(u.z) : 0.0f, ob ? hi(u.z) : 0.0f)};
+        const V3x2 q = add2(cc, mul2_kept(f2(c.w, c.w), nn, neg0));
+        p = V3x2{f2(ha ? lo(q.x) : lo(p.x), hb ? hi(q.x) : hi(p.x)), f2(ha ? lo(q.y) : lo(p.y), hb ? hi(q.y) : hi(p.y)),
+                 f2(ha ? lo(q.z) : lo(p.z), hb ? hi(q.z) : hi(p.z))};
+        pa |= ha;
+        pb |= hb;
+      }
+    }
+    if (pa | pb) {
+      const V3x2 g = sub2(p, st.w);
+      shift(pa, pb, g.x, st.D.x, st.s.x, s_next.x);
+      shift(pa, pb, g.y, st.D.y, st.s.y, s_next.y);
+      shift(pa, pb, g.z, st.D.z, st.s.z, s_next.z);
+    }
+  }
+  // A push by g: D and s by +g, the next segment by -g (at the tip there is
+  // none, and s_next is not used).
+  static __device__ __forceinline__ void shift(bool pa, bool pb, F2 g, F2& D, F2& s, F2& s_next) {
+    const F2 Dn = add2(D, g), sn = add2(s, g), nn = sub2(s_next, g);
+    D = f2(pa ? lo(Dn) : lo(D), pb ? hi(Dn) : hi(D));
+    s = f2(pa ? lo(sn) : lo(s), pb ? hi(sn) : hi(s));
+    s_next = f2(pa ? lo(nn) : lo(s_next), pb ? hi(nn) : hi(s_next));
+  }
+  __device__ __forceinline__ void store(int i, V3 s, V3 u, float rest) const {
+    X.store(i, f4(s, rest));
+    V.store(i, f4(u, vel_w<XS>(rest)));
+  }
+  // The velocity slot of a finished point: fma(-damping, e, D).
+  __device__ __forceinline__ V3 carry(V3 e, V3 D) const {
+    return V3{__fmaf_rn(K.neg_damping, e.x, D.x), __fmaf_rn(K.neg_damping, e.y, D.y),
+              __fmaf_rn(K.neg_damping, e.z, D.z)};
+  }
+  // One component of the points to link next: the pair's first stage takes
+  // (segment xs, u = vs), its second what the first finished (s, ua).
+  static __device__ __forceinline__ void next(F2& a, F2& d, float xs, float vs, float s, float ua, float f) {
+    const float da = __fadd_rn(vs, f), db = __fadd_rn(ua, f);
+    d = f2(da, db);
+    a = f2(__fadd_rn(xs, da), __fadd_rn(s, db));
+  }
+  __device__ __forceinline__ void advance(WaveStages& q, const WaveLinked& l, V3 x, V3 u, float rest, V3 ua) const {
+    next(q.a.x, q.d.x, x.x, u.x, lo(q.s.x), ua.x, K.h2F.x);
+    next(q.a.y, q.d.y, x.y, u.y, lo(q.s.y), ua.y, K.h2F.y);
+    next(q.a.z, q.d.z, x.z, u.z, lo(q.s.z), ua.z, K.h2F.z);
+    q.last_b = q.next_b;
+    q.next_b = q.last_a;
+    q.last_a = q.next_a;
+    q.next_a = rest;
+    q.s = l.s;
+    q.D = l.D;
+    q.w = l.w;
+  }
+  // Step i, 2 W <= i <= n - 2.
+  __device__ __forceinline__ void step(int i) {
+    const float4 vn = V.load(i + 1);
+    const float4 xn = with_rest<XS>(X.load(i + 1), vn);
+    WaveLinked l[P];
+#pragma unroll
+    for (int q = 0; q < P; ++q) l[q] = link(st[q]);
+    if (i - 1 >= jmin) {
+#pragma unroll
+      for (int q = 0; q < P; ++q)
+        if (F.flagged(st[q].w)) push(true, true, st[q], l[q].s);
+    }
+    store(i - (2 * W - 1), hi(st[P - 1].s), carry(hi(l[P - 1].e), hi(st[P - 1].D)), st[P - 1].last_b);
+#pragma unroll
+    for (int q = P - 1; q >= 0; --q) {
+      const V3 ua = carry(lo(l[q].e), lo(st[q].D));
+      if (q == 0) {
+        advance(st[0], l[0], xyz(xn), xyz(vn), xn.w, ua);
+      } else {
+        const WaveStages& o = st[q > 0 ? q - 1 : 0];
+        advance(st[q], l[q], hi(o.s), carry(hi(l[q > 0 ? q - 1 : 0].e), hi(o.D)), o.last_b, ua);
+      }
+    }
+  }
+  // Whether stage k tests the point it finishes in step t, and finishes one.
+  __device__ __forceinline__ bool tested(int tk, bool more, bool before) const {
+    return tk < 2 ? before && n - 2 + tk >= jmin : more && tk > 2 && tk - 2 >= jmin;
+  }
+  // Step t of the 2 W + 1 between sweeps r - 1 and r: stage k finishes its
+  // tip at t = 2 k + 1 and starts at t = 2 k + 2.
+  __device__ __forceinline__ void edge(int t, int r, int sweeps) {
+    const bool more = r < sweeps, before = r > 0;
+    if (t == 1) V.fence();  // points up to n - 2 W of sweep r - 1
+    float4 vn = make_float4(0.0f, 0.0f, 0.0f, 0.0f), xn = vn;
+    if (t >= 1 && more) {
+      vn = V.load(t);
+      xn = with_rest<XS>(X.load(t), vn);
+    }
+    if (more && t >= 2 && t % 2 == 0) {  // a stage starts: its leader is the root
+      const RootPath path{xyz(X.load(0)), xyz(V.load(0)), fc.substeps, fc.root_mode != HS_ROOT_PINNED};
+      const int ks = t / 2 - 1, k = k0 + W * r + ks;
+      const V3 rel = path.rel(k), D0 = sub(rel, path.rel(k - 1)), R = path.at(k, rel);
+#pragma unroll
+      for (int q = 0; q < P; ++q) {
+        if (ks == 2 * q) {
+          st[q].D = v3x2(D0, hi(st[q].D));
+          st[q].w = v3x2(R, hi(st[q].w));
+        }
+        if (ks == 2 * q + 1) {
+          st[q].D = v3x2(lo(st[q].D), D0);
+          st[q].w = v3x2(lo(st[q].w), R);
+        }
+      }
+    }
+    WaveLinked l[P];
+    V3 ua[P], ub[P];
+#pragma unroll
+    for (int q = 0; q < P; ++q) {
+      l[q] = link(st[q]);
+      const int ta = t - 4 * q, tb = ta - 2;  // the two stages' own steps
+      const bool testa = tested(ta, more, before), testb = tested(tb, more, before);
+      if ((testa || testb) && F.flagged(st[q].w)) push(testa, testb, st[q], l[q].s);
+      ua[q] = ta == 1 ? lo(st[q].D) : carry(lo(l[q].e), lo(st[q].D));  // a tip has no next correction
+      ub[q] = tb == 1 ? hi(st[q].D) : carry(hi(l[q].e), hi(st[q].D));
+    }
+    if (before && t < 2 * W) store(n - 2 * W + t, hi(st[P - 1].s), ub[P - 1], st[P - 1].last_b);
+#pragma unroll
+    for (int q = P - 1; q >= 0; --q) {
+      if (q == 0) {
+        advance(st[0], l[0], xyz(xn), xyz(vn), xn.w, ua[0]);
+      } else {
+        const WaveStages& o = st[q > 0 ? q - 1 : 0];
+        advance(st[q], l[q], hi(o.s), ub[q > 0 ? q - 1 : 0], o.last_b, ua[q]);
+      }
+    }
+    if (t == 2 * W) V.fence();  // the last points of sweep r - 1
+  }
+  __device__ __forceinline__ void run(int sweeps) {
+    const F2 z = f2(0.0f, 0.0f);
+    const V3x2 z3{z, z, z};
+#pragma unroll
+    for (int q = 0; q < P; ++q) st[q] = WaveStages{z3, z3, z3, z3, z3, 0.0f, 0.0f, 0.0f, 0.0f};
+    for (int r = 0; r <= sweeps; ++r) {
+      const int last = r < sweeps ? 2 * W : 2 * W - 1;
+#pragma unroll 1
+      for (int t = r == 0 ? 1 : 0; t <= last; ++t) edge(t, r, sweeps);
+      if (r < sweeps) {
+#pragma unroll 2
+        for (int i = 2 * W; i < n - 1; ++i) step(i);
+      }
+    }
+    V.fence();
+  }
+};
+
+// Substeps 0 .. k - 1 in sweeps of 2 P, then of 2; returns k. The others
+// (an odd last one, short strands) go one at a time (substeps_seg).
+template <int P, bool FAST, typename XS, typename VS, int NF>
+__device__ __forceinline__ int wave_substeps(const FrameConst& fc, const StrandConsts& K, const SphereFilter<NF>& F1,
+                                             const SphereSet& S, int n, int jmin, const XS& X, const VS& V) {
+  const SphereFilter2<NF> F(F1);
+  int k = 0;
+  if (P > 1 && n >= kWaveMinPoints<2 * P> && fc.substeps >= 2 * P) {
+    WavePass<P, FAST, XS, VS, NF> pass{K, fc, F, S, X, V, n, jmin, 0, negative_zero()};
+    pass.run(fc.substeps / (2 * P));
+    k = fc.substeps / (2 * P) * (2 * P);
+  }
+  if (n >= kWaveMinPoints<2> && fc.substeps - k >= 2) {
+    WavePass<1, FAST, XS, VS, NF> pass{K, fc, F, S, X, V, n, jmin, k, negative_zero()};
+    pass.run((fc.substeps - k) / 2);
+    k += (fc.substeps - k) / 2 * 2;
+  }
+  return k;
+}
+
 // ---- the frame ------------------------------------------------------------
 
 // Per-strand constants of a frame: force per unit mass, gravity
@@ -878,9 +1170,10 @@ __device__ __forceinline__ void substeps_seg(const FrameConst& fc, const StrandC
 // SPLIT: the DFTL pass shape (substep_single_pass_seg). One code shape per
 // kernel keeps the instruction cache warm: the batched kernels run one
 // loop; the plain step splits it.
-// PICK: the push-out's form (push_seg).
+// PICK: the push-out's form (push_seg). P: pairs of substeps at once
+// (WavePass; 0: one substep at a time). NF: slots of the sphere filter.
 template <bool REF, typename XS, typename VS, int M = kCachedSpheres, bool SPLIT = false, bool PICK = false,
-          bool FAST = false>
+          bool FAST = false, int P = 0, int NF = 8>
 __device__ __forceinline__ void strand_frame_stream(const FrameConst& fc, const SphereSet& S, const GroomView& g,
                                                     uint32_t s, bool active, const XS& X, const VS& V) {
   const int n = static_cast<int>(g.npoints);
@@ -925,7 +1218,7 @@ __device__ __forceinline__ void strand_frame_stream(const FrameConst& fc, const 
   V.fence();
 
   const StrandConsts K = strand_consts(fc, g, s, active);
-  const V3 target = root_target(fc, g, s, active, x0_start);
+  V3 target = root_target(fc, g, s, active, x0_start);
 
   // Spheres each strand can touch during the frame (see hs_step.cuh), and
   // the warp's first point that can touch one: point j stays within R_j (its
@@ -969,8 +1262,20 @@ __device__ __forceinline__ void strand_frame_stream(const FrameConst& fc, const 
         jmin = __reduce_min_sync(0xffffffffu, active ? jl : n);
       }
     }
-    const SphereFilter<8> F = filter_spheres<8>(S, reach, far);
-    substeps_seg<SPLIT, PICK, FAST>(fc, K, F, S, n, jmin, 0, x0_start, target, rest0, X, V);
+    const SphereFilter<NF> F = filter_spheres<NF>(S, reach, far);
+    int k0 = 0;  // substeps done in pairs
+    if constexpr (P > 0) {
+      // The root's path waits in slot 0.
+      X.store(0, f4(x0_start, rest0));
+      V.store(0, f4(target, rest0));
+      if (fc.iterations == 1) k0 = wave_substeps<P, FAST>(fc, K, F, S, n, jmin, X, V);
+      V.fence();
+      const float4 v0 = V.load(0);
+      x0_start = xyz(X.load(0));
+      target = xyz(v0);
+      rest0 = v0.w;
+    }
+    substeps_seg<SPLIT, PICK, FAST>(fc, K, F, S, n, jmin, k0, x0_start, target, rest0, X, V);
   }
 
   // Store: reference mode holds positions; DFTL mode rebuilds them from the
