@@ -21,6 +21,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -69,11 +70,12 @@ struct TessArgs {
 };
 
 // The shader's divisions, one table entry per distinct operand pair:
-// u = s / nsub, u / N, j / N, v = l / nlines (IEEE divisions, as the oracle).
+// u = s / nsub, u / N, j / N, v = l / nlines (IEEE divisions, as the oracle),
+// and the triangle sample of each (instance, line) pair.
 struct TessTables {
-  float4 basis[17];                                  // Hermite basis (c0..c3) at u = s / nsub
+  ulonglong2 basis[17][2];                           // Hermite basis at u = s / nsub: (c0, c0, c1, c1), (c2, c2, c3, c3)
   float rel[(HS_MAX_POINTS_PER_STRAND - 1) * 17];    // smoothstep(j / N + u / N), [j][s]
-  float v[16];                                       // l / nlines
+  float4 sample[16 * 16];                            // triangle sample (sx, sy, 1 - (sx + sy)), [instance][l]
 };
 
 __device__ __forceinline__ float dot4(float a0, float a1, float a2, float a3, float b0, float b1, float b2,
@@ -95,23 +97,51 @@ __device__ __forceinline__ float smoothstep01(float x);
 __device__ __forceinline__ void tess_tables(const TessArgs& a, TessTables& T) {
   const float n = static_cast<float>(a.npoints);
   const uint32_t ns = a.nsub + 1;
-  for (uint32_t k = threadIdx.x; k < ns; k += blockDim.x)
-    T.basis[k] = hermite_basis(__fdiv_rn(static_cast<float>(k), static_cast<float>(a.nsub)));
+  for (uint32_t k = threadIdx.x; k < ns; k += blockDim.x) {
+    const float4 c = hermite_basis(__fdiv_rn(static_cast<float>(k), static_cast<float>(a.nsub)));
+    T.basis[k][0] = make_ulonglong2(pair(c.x, c.x), pair(c.y, c.y));
+    T.basis[k][1] = make_ulonglong2(pair(c.z, c.z), pair(c.w, c.w));
+  }
   for (uint32_t k = threadIdx.x; k < (a.npoints - 1) * ns; k += blockDim.x) {
     const uint32_t j = k / ns, sub = k - j * ns;
     const float u = __fdiv_rn(static_cast<float>(sub), static_cast<float>(a.nsub));
     T.rel[k] = smoothstep01(__fadd_rn(__fdiv_rn(static_cast<float>(j), n), __fdiv_rn(u, n)));  // tes :65-66
   }
-  for (uint32_t k = threadIdx.x; k < a.nlines; k += blockDim.x)
-    T.v[k] = __fdiv_rn(static_cast<float>(k), static_cast<float>(a.nlines));
+  for (uint32_t k = threadIdx.x; k < a.ninstances * a.nlines; k += blockDim.x) {
+    const uint32_t inst = k / a.nlines, l = k - inst * a.nlines;
+    // gl_TessCoord v = l / nlines; the random offset (tes :55-58);
+    // randbuffer is vec3 under std430: element r starts at float 4r.
+    const float v = __fdiv_rn(static_cast<float>(l), static_cast<float>(a.nlines));
+    const int r = static_cast<int>(__fadd_rn(__fmul_rn(v, 40.0f), static_cast<float>(inst))) % HS_TESS_RANDOM_SIZE;
+    // sample_triangle2 (inc_maths.glsl:107-115); st.y is min(st.x, st.y)
+    // after st.x has become the max, i.e. st.y itself.
+    float sx = __ldg(a.random + 4 * r), sy = __ldg(a.random + 4 * r + 1);
+    if (__fadd_rn(sx, sy) > 1.0f) {
+      sx = fmaxf(sx, sy);
+      sy = fminf(sx, sy);
+      sx = __fsub_rn(1.0f, sx);
+    }
+    T.sample[k] = make_float4(sx, sy, __fsub_rn(1.0f, __fadd_rn(sx, sy)), 0.0f);
+  }
 }
+
+// A vector with its (x, y) as the halves of a two-wide instruction
+// (hs_device.cuh): each half rounds as the scalar operation does.
+struct P3 {
+  F2 xy;
+  float z;
+};
+// The basis at one u, each weight twice.
+struct Basis {
+  F2 c0, c1, c2, c3;
+};
 
 // hermite_mix (inc_maths.glsl:210-228): vU * mHermit * B, xyz only (the w
 // of the result is not used by the pass).
 // (...) * B with the basis c: B's columns (p0.x, p1.x, t0.x, t1.x) and so on.
-__device__ __forceinline__ float3 hermite(float3 p0, float3 p1, float3 t0, float3 t1, float4 c) {
-  return make_float3(dot4(c.x, c.y, c.z, c.w, p0.x, p1.x, t0.x, t1.x), dot4(c.x, c.y, c.z, c.w, p0.y, p1.y, t0.y, t1.y),
-                     dot4(c.x, c.y, c.z, c.w, p0.z, p1.z, t0.z, t1.z));
+__device__ __forceinline__ P3 hermite(P3 p0, P3 p1, P3 t0, P3 t1, const Basis& c) {
+  return P3{fma2(c.c3, t1.xy, fma2(c.c2, t0.xy, fma2(c.c1, p1.xy, mul2(c.c0, p0.xy)))),
+            dot4(lo(c.c0), lo(c.c1), lo(c.c2), lo(c.c3), p0.z, p1.z, t0.z, t1.z)};
 }
 
 // smoothstep2(0, 1, x) (inc_maths.glsl:263-266, maprange :239-241).
@@ -121,110 +151,127 @@ __device__ __forceinline__ float smoothstep01(float x) {
   return __fmul_rn(__fmul_rn(__fmul_rn(t, t), t), inner);
 }
 
-__device__ __forceinline__ float3 xyz3(float4 v) { return make_float3(v.x, v.y, v.z); }
-__device__ __forceinline__ float3 scaled(float4 v, float s) {
-  return make_float3(__fmul_rn(v.x, s), __fmul_rn(v.y, s), __fmul_rn(v.z, s));
-}
-
-// Blocks of 4 warps. The staging row of a line holds its nsub + 1 vertices
-// (each vertex ends one segment and starts the next, so the output row of
-// 2 nsub segment ends repeats them); 17 float4 a row, an odd stride, keep
-// the lanes' rows in different banks.
+// Blocks of 4 warps, a staging row of 2 nsub float4 a thread (the segment
+// ends of its line: vertex s ends segment s - 1 and starts segment s), one
+// float4 apart, so that the eight rows of a 128-bit store phase fall on
+// different banks.
 constexpr int kTessBlock = 128;
-constexpr int kTessRow = 17;
+__host__ __device__ constexpr uint32_t tess_row(uint32_t nsub) { return 2 * nsub + 1; }
+constexpr size_t tess_smem(uint32_t nsub) { return sizeof(float4) * kTessBlock * tess_row(nsub); }
 
-// One tessellation-evaluation vertex (tes_stream_hair.glsl:27-73) per
-// (line, u): the three strands' Hermite curves at the basis c, mixed by the
-// line's triangle sample (sx, sy, cz).
-__device__ __forceinline__ float4 tes_vertex(const float3 (&P)[6], const float3 (&T)[6], float4 c, float sx, float sy,
-                                             float cz, float rel) {
-  const float3 p0 = hermite(P[0], P[1], T[0], T[1], c);
-  const float3 p1 = hermite(P[2], P[3], T[2], T[3], c);
-  const float3 p2 = hermite(P[4], P[5], T[4], T[5], c);
-  const float x = __fmaf_rn(p2.x, cz, __fmaf_rn(p1.x, sy, __fmul_rn(p0.x, sx)));
-  const float y = __fmaf_rn(p2.y, cz, __fmaf_rn(p1.y, sy, __fmul_rn(p0.y, sx)));
-  const float z = __fmaf_rn(p2.z, cz, __fmaf_rn(p1.z, sy, __fmul_rn(p0.z, sx)));
-  return make_float4(x, y, z, rel);
+// A copy of `bytes` (a multiple of 16) from shared to global memory by the
+// copy engine, after this thread's writes to the source; the thread may
+// rewrite the source after copies_read(), and the copies are complete after
+// copies_done().
+__device__ __forceinline__ void copy_out(void* dst, const void* src, uint32_t bytes) {
+  const uint32_t from = static_cast<uint32_t>(__cvta_generic_to_shared(src));
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(from), "r"(bytes)
+               : "memory");
+  asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+__device__ __forceinline__ void copies_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void copies_done() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+
+// An isoline: line index = ((instance * nfaces + face) * (N - 1) + j) *
+// nlines + l.
+struct Isoline {
+  uint32_t l, j, face, inst;
+};
+__device__ __forceinline__ Isoline isoline(const TessArgs& a, uint64_t li, bool small) {
+  Isoline o;
+  if (small) {
+    const uint32_t l32 = static_cast<uint32_t>(li);
+    const uint32_t q1 = a.lines.div(l32);
+    o.l = l32 - q1 * a.nlines;
+    const uint32_t q2 = a.segs.div(q1);
+    o.j = q1 - q2 * (a.npoints - 1);
+    o.inst = a.faces_div.div(q2);
+    o.face = q2 - o.inst * a.nfaces;
+  } else {
+    uint64_t q = li;
+    o.l = static_cast<uint32_t>(q % a.nlines);
+    q /= a.nlines;
+    o.j = static_cast<uint32_t>(q % (a.npoints - 1));
+    q /= (a.npoints - 1);
+    o.face = static_cast<uint32_t>(q % a.nfaces);
+    o.inst = static_cast<uint32_t>(q / a.nfaces);
+  }
+  return o;
 }
 
-// A grid-stride loop over groups of 32 lines, one group per warp.
-// Line index = ((instance * nfaces + face) * (N - 1) + j) * nlines + l.
+// The patch (hair.cc:400-408): points j, j+1 of the triangle's strands.
+struct Patch {
+  float4 p[6], t[6];
+};
+__device__ __forceinline__ Patch gather(const TessArgs& a, const Isoline& o, uint3 f) {
+  Patch q;
+  const uint32_t strand[3] = {f.x, f.y, f.z};
+#pragma unroll
+  for (int k = 0; k < 6; ++k) {
+    const size_t idx = static_cast<size_t>(o.j + (k & 1)) * a.stride + strand[k >> 1];
+    q.p[k] = __ldg(a.pos + idx);
+    q.t[k] = __ldg(a.tangent + idx);
+  }
+  return q;
+}
+
+// A grid-stride loop over the isolines, one per thread.
+//
+// Bound by the writes (32 bytes a segment; a plain fill of as many bytes
+// takes 52 us). 736,920 lines of 16 segments (377 MB): with the rows
+// expanded and stored by the warp 83.7 us (57 M warp instructions, a third
+// of them the stores), as one bulk copy a line 73 to 78 us (26 M; the copies
+// alone 66 us, the evaluation alone 45); 338,688 lines of 7 segments 47.3 ->
+// 29 us. One copy a warp (rows without padding, each lane's vertices in
+// turn from another place) took 79.6 us, and the next line's gathers ahead
+// of the evaluation gained nothing.
 __global__ void __launch_bounds__(kTessBlock) k_tess(TessArgs a) {
+  extern __shared__ float4 stage[];  // [kTessBlock][tess_row(nsub)]
   __shared__ TessTables tab;
-  __shared__ float4 stage[kTessBlock / 32][32 * kTessRow];
   tess_tables(a, tab);
   __syncthreads();
-  const uint32_t warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-  float4* const st = stage[warp];
   const uint32_t ns = a.nsub + 1, row = 2 * a.nsub;
-  const uint64_t nlines_total = a.nvertices / ns;
-  const uint64_t groups = (nlines_total + 31) / 32;
-  const uint64_t step = static_cast<uint64_t>(gridDim.x) * (kTessBlock / 32);
-  for (uint64_t grp = static_cast<uint64_t>(blockIdx.x) * (kTessBlock / 32) + warp; grp < groups; grp += step) {
-    const uint64_t line0 = grp * 32;
-    const uint64_t li = line0 + lane;
-    if (li < nlines_total) {
-      uint32_t line, j, face, inst;
-      if (nlines_total <= 0xffffffffull) {
-        const uint32_t l32 = static_cast<uint32_t>(li);
-        const uint32_t q1 = a.lines.div(l32);
-        line = l32 - q1 * a.nlines;
-        const uint32_t q2 = a.segs.div(q1);
-        j = q1 - q2 * (a.npoints - 1);
-        inst = a.faces_div.div(q2);
-        face = q2 - inst * a.nfaces;
-      } else {
-        uint64_t q = li;
-        line = static_cast<uint32_t>(q % a.nlines);
-        q /= a.nlines;
-        j = static_cast<uint32_t>(q % (a.npoints - 1));
-        q /= (a.npoints - 1);
-        face = static_cast<uint32_t>(q % a.nfaces);
-        inst = static_cast<uint32_t>(q / a.nfaces);
-      }
-      // The patch (hair.cc:400-408): points j, j+1 of the triangle's strands.
-      const uint3 f = a.faces[face];
-      const uint32_t strand[3] = {f.x, f.y, f.z};
-      float3 P[6], T[6];
+  const uint64_t total = a.nvertices / ns;
+  const bool small = total <= 0xffffffffull;
+  const uint64_t step = static_cast<uint64_t>(gridDim.x) * kTessBlock;
+  float4* const mine = stage + threadIdx.x * tess_row(a.nsub);
+  const F2 scale = f2(a.scale, a.scale);
+  for (uint64_t li = static_cast<uint64_t>(blockIdx.x) * kTessBlock + threadIdx.x; li < total; li += step) {
+    const Isoline o = isoline(a, li, small);
+    const Patch q = gather(a, o, a.faces[o.face]);
+    P3 P[6], T[6];
 #pragma unroll
-      for (int k = 0; k < 6; ++k) {
-        const size_t idx = static_cast<size_t>(j + (k & 1)) * a.stride + strand[k >> 1];
-        P[k] = xyz3(__ldg(a.pos + idx));
-        T[k] = scaled(__ldg(a.tangent + idx), a.scale);  // tcs :41
-      }
-      // gl_TessCoord v = line / nlines; the random offset (tes :55-58);
-      // randbuffer is vec3 under std430: element r starts at float 4r.
-      const float v = tab.v[line];
-      const int r = static_cast<int>(__fadd_rn(__fmul_rn(v, 40.0f), static_cast<float>(inst))) % HS_TESS_RANDOM_SIZE;
-      // sample_triangle2 (inc_maths.glsl:107-115); st.y is min(st.x, st.y)
-      // after st.x has become the max, i.e. st.y itself.
-      float sx = __ldg(a.random + 4 * r), sy = __ldg(a.random + 4 * r + 1);
-      if (__fadd_rn(sx, sy) > 1.0f) {
-        sx = fmaxf(sx, sy);
-        sy = fminf(sx, sy);
-        sx = __fsub_rn(1.0f, sx);
-      }
-      const float cz = __fsub_rn(1.0f, __fadd_rn(sx, sy));
-      // The geometry shader's lines (gs :20-28): vertex s ends segment
-      // s - 1 and starts segment s (expanded when the rows are stored).
-      float4* const mine = st + lane * kTessRow;
-      const float* const rel = tab.rel + j * ns;
-      // Fully unrolled over the 17 possible vertices: independent vertices
-      // in flight (few warps fit an SM).
+    for (int k = 0; k < 6; ++k) {
+      P[k] = P3{f2(q.p[k].x, q.p[k].y), q.p[k].z};
+      T[k] = P3{mul2(f2(q.t[k].x, q.t[k].y), scale), __fmul_rn(q.t[k].z, a.scale)};  // tcs :41
+    }
+    const float4 st = tab.sample[o.inst * a.nlines + o.l];
+    const F2 sx2 = f2(st.x, st.x), sy2 = f2(st.y, st.y), cz2 = f2(st.z, st.z);
+    const float* const rel = tab.rel + o.j * ns;
+    copies_read();  // of this thread's last line
+    // One tessellation-evaluation vertex (tes_stream_hair.glsl:27-73) per
+    // (line, u): the three strands' Hermite curves, mixed by the triangle
+    // sample. Fully unrolled over the 17 possible vertices (a loop over fours
+    // takes 81 us).
 #pragma unroll
-      for (uint32_t sub = 0; sub < 17; ++sub) {
-        if (sub < ns) mine[sub] = tes_vertex(P, T, tab.basis[sub], sx, sy, cz, rel[sub]);
+    for (uint32_t sub = 0; sub < 17; ++sub) {
+      if (sub < ns) {
+        const ulonglong2 ca = tab.basis[sub][0], cb = tab.basis[sub][1];
+        const Basis c{F2{ca.x}, F2{ca.y}, F2{cb.x}, F2{cb.y}};
+        const P3 p0 = hermite(P[0], P[1], T[0], T[1], c);
+        const P3 p1 = hermite(P[2], P[3], T[2], T[3], c);
+        const P3 p2 = hermite(P[4], P[5], T[4], T[5], c);
+        const F2 xy = fma2(p2.xy, cz2, fma2(p1.xy, sy2, mul2(p0.xy, sx2)));
+        const float z = __fmaf_rn(p2.z, st.z, __fmaf_rn(p1.z, st.y, __fmul_rn(p0.z, st.x)));
+        const float4 vtx = make_float4(lo(xy), hi(xy), z, rel[sub]);
+        if (sub > 0) mine[2 * sub - 1] = vtx;
+        if (sub < a.nsub) mine[2 * sub] = vtx;
       }
     }
-    __syncwarp();
-    // The warp's lines are contiguous in the output: row by row, coalesced;
-    // segment end k of a line is its vertex (k + 1) / 2.
-    const uint64_t nl = min(static_cast<uint64_t>(32), nlines_total - line0);
-    float4* const out = a.out + line0 * row;
-    for (uint32_t l = 0; l < nl; ++l)
-      for (uint32_t k = lane; k < row; k += 32) out[static_cast<size_t>(l) * row + k] = st[l * kTessRow + (k + 1) / 2];
-    __syncwarp();
+    copy_out(a.out + li * row, mine, row * static_cast<uint32_t>(sizeof(float4)));
   }
+  copies_done();
 }
 
 }  // namespace
@@ -360,16 +407,22 @@ HS_API hs_status hs_tess_stream(hs_groom* g, const hs_tess_params* p, uint64_t* 
   a.segs = FastDiv::make(g->npoints - 1);
   a.faces_div = FastDiv::make(g->tess_nfaces);
   // One wave of resident blocks: each builds the tables once.
+  static std::atomic<uint64_t> optin{0};
+  once_per_device(optin, [] {
+    cudaFuncSetAttribute(k_tess, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         static_cast<int>(tess_smem(16)));
+  });
+  const size_t smem = tess_smem(p->nsubsegments);
   int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tess, kTessBlock, 0) != cudaSuccess) {
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tess, kTessBlock, smem) != cudaSuccess) {
     cudaGetLastError();
     per_sm = 1;
   }
   const uint64_t resident = static_cast<uint64_t>(std::max(1, per_sm)) *
                             static_cast<uint64_t>(device_attribute(cudaDevAttrMultiProcessorCount, 1));
-  const uint64_t groups = (a.nvertices / (p->nsubsegments + 1) + 31) / 32;
-  const uint64_t blocks = std::min<uint64_t>((groups + kTessBlock / 32 - 1) / (kTessBlock / 32), resident);
-  k_tess<<<static_cast<unsigned>(std::max<uint64_t>(blocks, 1)), kTessBlock, 0, s>>>(a);
+  const uint64_t lines = a.nvertices / (p->nsubsegments + 1);
+  const uint64_t blocks = std::min<uint64_t>((lines + kTessBlock - 1) / kTessBlock, resident);
+  k_tess<<<static_cast<unsigned>(std::max<uint64_t>(blocks, 1)), kTessBlock, smem, s>>>(a);
   e = cudaGetLastError();
   g->ctx->launches += 1;
   if (e != cudaSuccess) return cuda_fail(e, "hs_tess_stream: launch");
