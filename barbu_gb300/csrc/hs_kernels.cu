@@ -71,8 +71,12 @@ struct PlainVsmem {
 
 // FAST (every kernel below): the groom's FAST contract, a kernel of its own
 // (no code of the other contract in it).
+// Reference mode is held to 80 registers (the frame's constants of 8 points
+// spill 88 bytes), so that 11 blocks fit an SM rather than 10: 100,003
+// strands x 8 alone 26.5 -> 21.2 us (their 1,563 blocks are then one wave),
+// three such grooms in turn 14.9 -> 14.4 us.
 template <int CAP, bool REF, bool FAST>
-__global__ void __launch_bounds__(kStepBlock) k_step(GroomView g, FrameConst fc) {
+__global__ void __launch_bounds__(kStepBlock, REF ? 11 : 0) k_step(GroomView g, FrameConst fc) {
   extern __shared__ float4 s_vel[];  // per-thread velocity rows, when in shared memory
   __shared__ float4 s_c[HS_MAX_SPHERES];
   __shared__ float s_r2[HS_MAX_SPHERES];

@@ -108,6 +108,62 @@ constexpr size_t vslot_bytes(int threads) {
 __device__ __forceinline__ float4 f4(V3 a, float w) { return make_float4(a.x, a.y, a.z, w); }
 __device__ __forceinline__ V3 xyz(float4 a) { return v3(a.x, a.y, a.z); }
 
+// One constraint iteration. Each iteration sets every velocity anew, so only
+// a substep's last one does (VEL): 100,003 strands of 8 points, 8 iterations,
+// three grooms in turn 15.9 -> 14.2 us with k_step's register bound (bound by instruction issue, then by
+// memory: the frame's bytes take 7.5). Two iterations at once, or the
+// collisions of two points at once, as halves of two-wide instructions need
+// 116 to 136 registers where this takes 95, and come out at 15.8 to 23.6 us.
+template <int CAP, bool VEL, typename VST>
+__device__ __forceinline__ void ref_iteration(const FrameConst& fc, const SphereSet& S, int n, uint32_t reach,
+                                              V3 (&X)[CAP], VST& vs) {
+  // DistanceConstraint (:109-121): follow the leader, root to tip.
+  V3 nprev = v3(0.0f, -1.0f, 0.0f);
+#pragma unroll
+  for (int i = 1; i < CAP; ++i) {
+    if (i < n) {
+      const float rest_i = vs.get_w(i);
+      const V3 p1 = X[i];
+      const V3 d = sub(p1, X[i - 1]);
+      const float d2 = dot(d, d);
+      const V3 nd = d2 > 0.0f ? mul(d, inversesqrt(d2)) : nprev;
+      nprev = nd;
+      X[i] = add(X[i - 1], mul(__fmul_rn(fc.length_scale, rest_i), nd));
+      if constexpr (VEL) {
+        // :116 then :119-121: each point takes its own correction and the
+        // next link replaces it with the next point's, damped; the tip,
+        // last in the chain, keeps its own.
+        const V3 corr = sub(X[i], p1);
+        vs.set(i, f4(corr, rest_i));
+        if (i >= 2) vs.set(i - 1, f4(mul(corr, fc.damping), vs.get_w(i - 1)));
+      }
+    }
+  }
+  // CollisionConstraint (:149-153): every point but the root, each
+  // against the reachable spheres in index order (CollideSphere, :129-139).
+  for (uint32_t todo = reach; todo; todo &= todo - 1u) {
+    const int k = __ffs(todo) - 1;
+    const float4 c = S.c[k];
+    const float r2 = S.r2[k];
+    const V3 cc = v3(c.x, c.y, c.z);
+#pragma unroll
+    for (int i = 1; i < CAP; ++i) {
+      if (i < n) {
+        const V3 pt = sub(X[i], cc);
+        const float dp = dot(pt, pt);
+        if (dp < r2) {
+          const V3 nn = dp > 0.0f ? mul(pt, inversesqrt(dp)) : v3(0.0f, 1.0f, 0.0f);
+          X[i] = add(cc, mul(c.w, nn));
+          if constexpr (VEL) {
+            const float4 sl = vs.get(i);
+            vs.set(i, f4(reflect(xyz(sl), nn), sl.w));  // :137
+          }
+        }
+      }
+    }
+  }
+}
+
 // One frame of strand s in reference mode. CAP: compile-time capacity
 // (register arrays); n = g.npoints <= CAP at run time (uniform across the
 // groom). VSMEM: where the velocity slots live; vs_rows/thread: the block's
@@ -196,53 +252,8 @@ __device__ __forceinline__ void strand_frame_ref(const FrameConst& fc, const Sph
       }
     }
 
-    for (int it = 0; it < fc.iterations; ++it) {
-      // DistanceConstraint (:109-121): follow the leader, root to tip.
-      V3 nprev = v3(0.0f, -1.0f, 0.0f);
-      float rest_prev = 0.0f;
-#pragma unroll
-      for (int i = 1; i < CAP; ++i) {
-        if (i < n) {
-          const float rest_i = vs.get_w(i);
-          const V3 p1 = X[i];
-          const V3 d = sub(p1, X[i - 1]);
-          const float d2 = dot(d, d);
-          const V3 nd = d2 > 0.0f ? mul(d, inversesqrt(d2)) : nprev;
-          nprev = nd;
-          X[i] = add(X[i - 1], mul(__fmul_rn(fc.length_scale, rest_i), nd));
-          const V3 corr = sub(X[i], p1);
-          // :116 then :119-121: each point takes its own correction and
-          // the next link replaces it with the next point's, damped; the
-          // tip, last in the chain, keeps its own.
-          vs.set(i, f4(corr, rest_i));
-          if (i >= 2) vs.set(i - 1, f4(mul(corr, fc.damping), rest_prev));
-          rest_prev = rest_i;
-        }
-      }
-      // CollisionConstraint (:149-153): every point but the root, each
-      // against the reachable spheres in index order (CollideSphere, :129-139).
-      uint32_t todo = reach;
-      while (todo) {
-        const int kk = __ffs(todo) - 1;
-        todo &= todo - 1u;
-        const float4 c = S.c[kk];
-        const float r2 = S.r2[kk];
-        const V3 cc = v3(c.x, c.y, c.z);
-#pragma unroll
-        for (int i = 1; i < CAP; ++i) {
-          if (i < n) {
-            const V3 pt = sub(X[i], cc);
-            const float dp = dot(pt, pt);
-            if (dp < r2) {
-              const V3 nn = dp > 0.0f ? mul(pt, inversesqrt(dp)) : v3(0.0f, 1.0f, 0.0f);
-              X[i] = add(cc, mul(c.w, nn));
-              const float4 sl = vs.get(i);
-              vs.set(i, f4(reflect(xyz(sl), nn), sl.w));  // :137
-            }
-          }
-        }
-      }
-    }
+    for (int it = 1; it < fc.iterations; ++it) ref_iteration<CAP, false>(fc, S, n, reach, X, vs);
+    ref_iteration<CAP, true>(fc, S, n, reach, X, vs);
     const float4 s0 = vs.get(0);
     vs.set(0, f4(sub(X[0], x0_old), s0.w));  // :192
   }
