@@ -1,5 +1,6 @@
 // hs_kernels.cu -- the per-groom kernels: step, init, layout transposes.
 #include <algorithm>
+#include <type_traits>
 
 #include "hs_internal.h"
 #include "hs_lanes.cuh"
@@ -319,52 +320,71 @@ __global__ void k_init(GroomView g, InitArgs a, float4* root_rest) {
 // at strand-major row order[s]: the outside sees the caller's order.
 constexpr int kTileStrands = 32;
 
-// Tile rows are padded by one float4 so that the 32 strands of a point
-// (one row each) fall in different shared-memory banks.
-__global__ void k_to_strand_major(const float4* __restrict__ soa, float4* __restrict__ out,
-                                  const uint32_t* __restrict__ order, uint32_t nstrands, uint32_t npoints,
-                                  uint32_t stride) {
-  __shared__ float4 tile[kTileStrands * (HS_MAX_POINTS_PER_STRAND + 1)];
-  const uint32_t s0 = blockIdx.x * kTileStrands;
+// C: floats a point in `out`: 4, or 3 for (x, y, z) alone. Bound by memory
+// latency (a block is one round of loads, a barrier, one of stores), so the
+// strands' places are loaded with their points, not after the barrier; no
+// index is divided by N, and tile rows are an odd number of float4, so that
+// the eight strands of a 128-bit store phase fall in different banks. A warp
+// writes `per` strands at a time (a power of two; one above 16 points).
+// Before (places after the barrier, t / N per point, rows of N + 1): 50,021
+// strands x 23 10.5 -> 7.9 us, 65,536 x 16 8.3 -> 7.4, 262,144 x 32 58 -> 52
+// (268 MB moved, 40 us at the copy bandwidth). Blocks of 4 warps up to 12
+// points a strand, of 8 above (4 against 8 warps, 100,003 x 9: 6.3 against
+// 8.3 us; 50,021 x 23: 8.3 against 7.7; 20,000 x 64: 9.4 against 8.4). Rows handed to the copy engine: 47 us for 262,144 x 32, but 8.3 for
+// 50,021 x 23 and 5.3 against 4.2 for 4,096 x 16.
+template <int C>
+__global__ void __launch_bounds__(256) k_to_strand_major(const float4* __restrict__ soa, float* __restrict__ out,
+                                                         const uint32_t* __restrict__ order, uint32_t nstrands,
+                                                         uint32_t npoints, uint32_t stride, uint32_t row, uint32_t per) {
+  extern __shared__ float4 tile[];  // [kTileStrands][row]
+  using Elem = typename std::conditional<C == 4, float4, float>::type;
+  const uint32_t s0 = blockIdx.x * kTileStrands, lane = threadIdx.x % 32, warp = threadIdx.x / 32;
   const uint32_t ns = min(static_cast<uint32_t>(kTileStrands), nstrands - s0);
-  const uint32_t total = ns * npoints;
-  const uint32_t row = npoints + 1;
-  for (uint32_t t = threadIdx.x; t < kTileStrands * npoints; t += blockDim.x) {
-    const uint32_t i = t / kTileStrands, sl = t % kTileStrands;
-    if (sl < ns) tile[sl * row + i] = soa[static_cast<size_t>(i) * stride + s0 + sl];
+  const uint32_t place = lane < ns ? order[s0 + lane] : 0u;
+  if (lane < ns) {
+    const float4* const from = soa + s0 + lane;
+#pragma unroll 4
+    for (uint32_t i = warp; i < npoints; i += blockDim.x / 32) tile[lane * row + i] = from[static_cast<size_t>(i) * stride];
   }
   __syncthreads();
-  for (uint32_t t = threadIdx.x; t < total; t += blockDim.x) {
-    const uint32_t sl = t / npoints, i = t % npoints;
-    out[static_cast<size_t>(order[s0 + sl]) * npoints + i] = tile[sl * row + i];
-  }
-}
-
-// The same transpose to (x, y, z) only, 12 bytes a point. Block 32 x 8:
-// a warp writes 32 consecutive points of one strand (384 contiguous bytes
-// in three 4-byte stores a thread), with no division in the index math.
-__global__ void k_to_strand_major_xyz(const float4* __restrict__ soa, float* __restrict__ out,
-                                      const uint32_t* __restrict__ order, uint32_t nstrands, uint32_t npoints,
-                                      uint32_t stride) {
-  __shared__ float4 tile[kTileStrands * (HS_MAX_POINTS_PER_STRAND + 1)];
-  const uint32_t s0 = blockIdx.x * kTileStrands;
-  const uint32_t ns = min(static_cast<uint32_t>(kTileStrands), nstrands - s0);
-  const uint32_t row = npoints + 1;
-  const uint32_t sl_in = threadIdx.x;  // strand of the tile, loads
-  for (uint32_t i = threadIdx.y; i < npoints; i += blockDim.y)
-    if (sl_in < ns) tile[sl_in * row + i] = soa[static_cast<size_t>(i) * stride + s0 + sl_in];
-  __syncthreads();
-  for (uint32_t sl = threadIdx.y; sl < ns; sl += blockDim.y) {
-    float* o = out + static_cast<size_t>(order[s0 + sl]) * 3 * npoints;
-    for (uint32_t i = threadIdx.x; i < npoints; i += blockDim.x) {
-      const float4 p = tile[sl * row + i];
-      o[3 * i] = p.x;
-      o[3 * i + 1] = p.y;
-      o[3 * i + 2] = p.z;
+  const uint32_t elems = C == 4 ? npoints : 3 * npoints, warps = blockDim.x / 32;
+  const auto put = [&](uint32_t sl, uint32_t to, uint32_t e) {
+    const float4* const r = tile + sl * row;
+    Elem* const o = reinterpret_cast<Elem*>(out) + static_cast<size_t>(to) * elems;
+    if constexpr (C == 4) o[e] = r[e];
+    else o[e] = reinterpret_cast<const float*>(r)[e + e / 3];
+  };
+  if (per == 1) {
+#pragma unroll 2
+    for (uint32_t sl = warp; sl < ns; sl += warps) {
+      const uint32_t to = __shfl_sync(0xffffffffu, place, sl);
+      for (uint32_t e = lane; e < elems; e += 32) put(sl, to, e);
+    }
+  } else {  // elems <= 32 / per
+    const uint32_t width = 32 / per, e = lane % width;
+#pragma unroll 2
+    for (uint32_t b = warp * per; b < kTileStrands; b += warps * per) {
+      const uint32_t sl = b + lane / width;
+      const uint32_t to = __shfl_sync(0xffffffffu, place, sl);
+      if (sl < ns && e < elems) put(sl, to, e);
     }
   }
 }
 
+template <int C>
+cudaError_t launch_strand_major(const float4* soa, float* out, const uint32_t* order, uint32_t nstrands,
+                                uint32_t npoints, uint32_t stride, cudaStream_t st) {
+  if (nstrands == 0) return cudaSuccess;
+  const uint32_t row = npoints | 1u, elems = C == 4 ? npoints : 3 * npoints;
+  uint32_t per = 1;
+  while (per < 32 && 2 * per * elems <= 32) per *= 2;
+  k_to_strand_major<C><<<(nstrands + kTileStrands - 1) / kTileStrands, npoints <= 12 ? 128 : 256,
+                         sizeof(float4) * kTileStrands * row, st>>>(soa, out, order, nstrands, npoints, stride, row, per);
+  return cudaGetLastError();
+}
+
+// Tile rows are padded by one float4 so that the 32 strands of a point
+// (one row each) fall in different shared-memory banks.
 __global__ void k_from_strand_major(const float4* __restrict__ in, float4* __restrict__ soa,
                                     const uint32_t* __restrict__ order, uint32_t nstrands, uint32_t npoints,
                                     uint32_t stride) {
@@ -453,18 +473,12 @@ cudaError_t launch_init(const GroomView& g, const InitArgs& a, float4* root_rest
 
 cudaError_t launch_to_strand_major(const float4* soa, float4* out, const uint32_t* order, uint32_t nstrands,
                                    uint32_t npoints, uint32_t stride, cudaStream_t st) {
-  if (nstrands == 0) return cudaSuccess;
-  k_to_strand_major<<<(nstrands + kTileStrands - 1) / kTileStrands, 256, 0, st>>>(soa, out, order, nstrands,
-                                                                                    npoints, stride);
-  return cudaGetLastError();
+  return launch_strand_major<4>(soa, reinterpret_cast<float*>(out), order, nstrands, npoints, stride, st);
 }
 
 cudaError_t launch_to_strand_major_xyz(const float4* soa, float* out, const uint32_t* order, uint32_t nstrands,
                                        uint32_t npoints, uint32_t stride, cudaStream_t st) {
-  if (nstrands == 0) return cudaSuccess;
-  k_to_strand_major_xyz<<<(nstrands + kTileStrands - 1) / kTileStrands, dim3(kTileStrands, 8), 0, st>>>(
-      soa, out, order, nstrands, npoints, stride);
-  return cudaGetLastError();
+  return launch_strand_major<3>(soa, out, order, nstrands, npoints, stride, st);
 }
 
 cudaError_t launch_from_strand_major(const float4* in, float4* soa, const uint32_t* order, uint32_t nstrands,
