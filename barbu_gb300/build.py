@@ -1,6 +1,7 @@
 """Build the hair-simulation library in tree.
 
-barbu_gb300/csrc/*.cu -> barbu_gb300/lib/libhairsim.so, for sm_103a only.
+barbu_gb300/csrc/*.cu -> barbu_gb300/lib/libhairsim.so, for sm_103a only, and
+the binding's call module, csrc/hs_pycalls.c -> barbu_gb300/_hscalls.so.
 One nvcc process per translation unit, in parallel, then one link. Host code
 is compiled without floating-point contraction so host-side parameter
 arithmetic rounds like the device's.
@@ -12,6 +13,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
@@ -19,6 +21,7 @@ CSRC = os.path.join(HERE, "csrc")
 BUILD = os.path.join(HERE, "_build")
 LIB_DIR = os.path.join(HERE, "lib")
 LIB = os.path.join(LIB_DIR, "libhairsim.so")
+CALLS = os.path.join(HERE, "_hscalls.so")
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 
 
@@ -46,6 +49,17 @@ def _compile(src: str, verbose_ptxas: bool) -> str:
     return obj
 
 
+def build_calls() -> str:
+    tmp = CALLS + ".tmp"
+    cmd = [shutil.which("gcc") or "cc", "-O2", "-fPIC", "-shared", "-fvisibility=hidden", "-Wall", "-I",
+           sysconfig.get_paths()["include"], os.path.join(CSRC, "hs_pycalls.c"), "-o", tmp]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"building {CALLS} failed:\n{r.stdout}\n{r.stderr}")
+    os.replace(tmp, CALLS)
+    return CALLS
+
+
 def build(verbose_ptxas: bool = False) -> str:
     os.makedirs(BUILD, exist_ok=True)
     os.makedirs(LIB_DIR, exist_ok=True)
@@ -58,6 +72,7 @@ def build(verbose_ptxas: bool = False) -> str:
     if r.returncode != 0:
         raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
     os.replace(tmp, LIB)
+    build_calls()
     return LIB
 
 

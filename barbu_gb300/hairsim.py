@@ -21,6 +21,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "lib", "libhairsim.so")
 
 _lib = None
+_calls = None  # the per-frame calls without ctypes (csrc/hs_pycalls.c)
 
 
 class HairSimError(RuntimeError):
@@ -102,15 +103,45 @@ def _declare(L):
 
 def lib():
     """Loads libhairsim.so (raises if it has not been built)."""
-    global _lib
+    global _lib, _calls
     if _lib is None:
         if not os.path.exists(LIB_PATH):
             raise ImportError(f"{LIB_PATH} is missing: build it with `python -m barbu_gb300.build` "
                               "(the library has no CPU fallback)")
+        from . import _hscalls  # built with the library
         L = C.CDLL(LIB_PATH)
         _declare(L)
+        for name in _ADDRESS:
+            _ADDRESS[name] = C.cast(getattr(L, name), C.c_void_p).value
+        _calls = _hscalls
         _lib = L
     return _lib
+
+
+# Addresses of the functions the per-frame methods call through _calls (both
+# filled when the library is loaded, which precedes any handle).
+_ADDRESS = dict.fromkeys(("hs_update", "hs_set_bounding_sphere", "hs_set_wind", "hs_set_root_transform",
+                          "hs_set_spheres", "hs_set_bone_matrices"))
+
+
+def _call_floats(name, handle, a, count):
+    """Status of name(handle, array of `count` floats)."""
+    st = _calls.floats(_ADDRESS[name], handle, a, count)
+    if st is None:
+        a = _f32(a, count)
+        st = getattr(lib(), name)(handle, _ptr(a))
+    if st:
+        check(st, name)
+
+
+def _call_rows(name, handle, a, width):
+    """Status of name(handle, rows of `width` floats, number of rows)."""
+    st = _calls.rows(_ADDRESS[name], handle, a, width)
+    if st is None:
+        a = _f32(a).reshape(-1, width)
+        st = getattr(lib(), name)(handle, _ptr(a), a.shape[0])
+    if st:
+        check(st, name)
 
 
 def marschner_params_reference() -> abi.MarschnerParams:
@@ -308,20 +339,16 @@ class Groom:
         check(lib().hs_groom_set_params(self.h, C.byref(sim)), "hs_groom_set_params")
 
     def set_bounding_sphere(self, xyzr):
-        a = _f32(xyzr, 4)
-        check(lib().hs_set_bounding_sphere(self.h, _ptr(a)), "hs_set_bounding_sphere")
+        _call_floats("hs_set_bounding_sphere", self.h, xyzr, 4)
 
     def set_spheres(self, xyzr):
-        a = _f32(xyzr).reshape(-1, 4)
-        check(lib().hs_set_spheres(self.h, _ptr(a), a.shape[0]), "hs_set_spheres")
+        _call_rows("hs_set_spheres", self.h, xyzr, 4)
 
     def set_wind(self, w):
-        a = _f32(w, 3)
-        check(lib().hs_set_wind(self.h, _ptr(a)), "hs_set_wind")
+        _call_floats("hs_set_wind", self.h, w, 3)
 
     def set_root_transform(self, m):
-        a = _f32(m, 16)
-        check(lib().hs_set_root_transform(self.h, _ptr(a)), "hs_set_root_transform")
+        _call_floats("hs_set_root_transform", self.h, m, 16)
 
     def set_roots(self, xyz):
         a = _f32(xyz, 3 * self.nstrands)
@@ -343,8 +370,7 @@ class Groom:
 
     def set_bone_matrices(self, m):
         """hs_set_bone_matrices: (nbones, 16) rigid column-major skinning matrices."""
-        a = _f32(m).reshape(-1, 16)
-        check(lib().hs_set_bone_matrices(self.h, _ptr(a), a.shape[0]), "hs_set_bone_matrices")
+        _call_rows("hs_set_bone_matrices", self.h, m, 16)
 
     def stats(self) -> dict | None:
         """hs_groom_stats: bounds, kinetic energy and largest speed of the
@@ -386,7 +412,11 @@ class Groom:
         return out
 
     def update(self, dt: float):
-        check(lib().hs_update(self.h, dt), "hs_update")
+        st = _calls.frame(_ADDRESS["hs_update"], self.h, dt)
+        if st is None:
+            st = lib().hs_update(self.h, dt)
+        if st:
+            check(st, "hs_update")
 
     def readback(self, out=None) -> np.ndarray:
         """Positions (x, y, z, restlength), shape (nstrands, npoints, 4)."""
@@ -502,7 +532,7 @@ class Hair:
         return self.nroots != 0
 
     def set_bounding_sphere(self, xyzr):
-        self._bsphere = np.asarray(xyzr, np.float32).reshape(4).copy()
+        self._bsphere = np.array(xyzr, np.float32).reshape(4)
 
     def update(self, dt: float):
         if not self.initialized():
