@@ -14,11 +14,6 @@ namespace {
 
 constexpr int kStepBlock = 64;
 
-// AUTO mapping of the plain step: lane groups while they make at most this
-// many warps per SM (32-strand tiles x lanes per strand) for strands of up
-// to 16 points, proportionally more for longer strands.
-constexpr int kLanesWarpsPerSm = 16;
-
 // Overlapped frames (programmatic dependent launch). A groom's frames are
 // back-to-back kernels on one stream; launched by launch_overlapped, a
 // frame's blocks may become resident while the previous kernel's last
@@ -132,11 +127,10 @@ __global__ void __launch_bounds__(kStreamBlock) k_step_stream(GroomView g, Frame
 // TMEM velocity slots).
 constexpr int kTmemBlock = 128;
 
-// MANY: the push-out's form for grooms among many spheres (push_seg). LONG:
-// more than 32 points, where tensor memory holds two blocks an SM: four
-// substeps at once (WavePass).
-template <bool REF, bool MANY, bool LONG, bool FAST>
-__global__ void __launch_bounds__(kTmemBlock, LONG ? 2 : 4) k_step_stream_tmem(GroomView g, FrameConst fc) {
+// MANY: the push-out's form for grooms among many spheres (push_seg). P:
+// pairs of substeps at once (step_pairs, WavePass).
+template <bool REF, bool MANY, int P, bool FAST>
+__global__ void __launch_bounds__(kTmemBlock, P == 2 ? 2 : 4) k_step_stream_tmem(GroomView g, FrameConst fc) {
   extern __shared__ float4 s_pos[];  // positions, compact: float2 (x, y) then float z, each [npoints][kTmemBlock]
   __shared__ float4 s_c[HS_MAX_SPHERES];
   __shared__ float s_r2[HS_MAX_SPHERES];
@@ -160,7 +154,7 @@ __global__ void __launch_bounds__(kTmemBlock, LONG ? 2 : 4) k_step_stream_tmem(G
   float2* xy = reinterpret_cast<float2*>(s_pos);
   float* z = reinterpret_cast<float*>(xy + g.npoints * kTmemBlock);
   const XShared3 X{xy + threadIdx.x, z + threadIdx.x, kTmemBlock};
-  strand_frame_stream<REF, XShared3, VTmem, 8, true, MANY, FAST, LONG ? 2 : 0>(fc, S, g, s, s < g.nstrands, X, V);
+  strand_frame_stream<REF, XShared3, VTmem, 8, true, MANY, FAST, P, P == 1 ? 4 : 8>(fc, S, g, s, s < g.nstrands, X, V);
   tmem::fence_before_sync();
   __syncthreads();
   tmem::fence_after_sync();
@@ -184,11 +178,41 @@ size_t tmem_step_smem(uint32_t npoints) {
 // push-out goes through all of those (measured at 7 and 16: push_seg).
 constexpr int kFewSpheres = 8;
 
+// Pairs of substeps a DFTL groom runs at once. They pay where schedulers wait
+// on chain links: less than a wave of warps (16 an SM, 8 for more than 32
+// points), longer strands, sphere tests to run two-wide. Single pass against
+// one pair / two pairs, us a frame, 8 substeps (EXACT; FAST gains a few percent
+// less):
+//   less than a wave  60,000 x 32 among 7 spheres 48.5 / 42.8, among 32 126 /
+//                     93; 60,000 x 16 among 24 48.9 / 42.0; 50,021 x 12 among
+//                     7 16.5 / 17.2; 38,133 x 32 without 10.8 / 11.9 (S 4);
+//                     20,000 x 36 among 8 47.7 / 35.5 / 36.6
+//   more              262,144 x 32 among 7 125 / 131; 150,000 x 36 among 4 111
+//                     / 113 / 117; 150,000 x 64 among 4 180 / 175 / 172, among
+//                     32 401 / 392 / 343
+//   one sphere        60,000 x 32 (FAST) 37.1 / 37.7; 150,000 x 64 253 / 225 /
+//                     229 (a head: every strand is near it)
+//   none              150,000 x 36 97 / 103 / 104, x 64 159 / 159 / 153
+int step_pairs(const GroomView& g, const FrameConst& fc) {
+  if (fc.iterations != 1 || fc.substeps < 2) return 0;
+  const bool is_long = g.npoints > 32;
+  const uint32_t sms = static_cast<uint32_t>(device_attribute(cudaDevAttrMultiProcessorCount, 152));
+  const bool wave = (g.nstrands + 31) / 32 <= (is_long ? 8u : 16u) * sms;
+  if (!is_long) return wave && fc.nspheres > 1 && (g.npoints > 20 || fc.nspheres > 16) ? 1 : 0;
+  if (fc.nspheres == 0) return g.npoints > 48 ? 2 : 0;
+  if (fc.nspheres == 1 || wave) return 1;
+  return fc.nspheres > 8 || g.npoints > 48 ? 2 : 0;
+}
+
 using TmemStep = void (*)(GroomView, FrameConst);
-TmemStep dftl_step_tmem(bool many, bool is_long, bool fast) {
-  if (is_long) return fast ? k_step_stream_tmem<false, false, true, true> : k_step_stream_tmem<false, false, true, false>;
-  if (many) return fast ? k_step_stream_tmem<false, true, false, true> : k_step_stream_tmem<false, true, false, false>;
-  return fast ? k_step_stream_tmem<false, false, false, true> : k_step_stream_tmem<false, false, false, false>;
+template <bool FAST>
+TmemStep dftl_step_tmem(bool many, int pairs) {
+  if (pairs == 2) return k_step_stream_tmem<false, false, 2, FAST>;
+  if (pairs == 1) return k_step_stream_tmem<false, false, 1, FAST>;
+  return many ? k_step_stream_tmem<false, true, 0, FAST> : k_step_stream_tmem<false, false, 0, FAST>;
+}
+TmemStep dftl_step_tmem(bool many, int pairs, bool fast) {
+  return fast ? dftl_step_tmem<true>(many, pairs) : dftl_step_tmem<false>(many, pairs);
 }
 
 cudaError_t launch_step_stream_tmem(const GroomView& g, const FrameConst& fc, cudaStream_t st) {
@@ -199,14 +223,13 @@ cudaError_t launch_step_stream_tmem(const GroomView& g, const FrameConst& fc, cu
     const int bytes = 200 * 1024;
     for (const bool fast : {false, true})
       for (const bool many : {false, true})
-        for (const bool is_long : {false, true})
-          cudaFuncSetAttribute(dftl_step_tmem(many, is_long, fast), cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    cudaFuncSetAttribute(k_step_stream_tmem<true, false, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         bytes);
+        for (const int pairs : {0, 1, 2})
+          cudaFuncSetAttribute(dftl_step_tmem(many, pairs, fast), cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    cudaFuncSetAttribute(k_step_stream_tmem<true, false, 0, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
   });
   if (fc.mode == HS_MODE_REFERENCE)
-    return launch_overlapped(k_step_stream_tmem<true, false, false, false>, grid, kTmemBlock, smem, st, g, fc);
-  return launch_overlapped(dftl_step_tmem(fc.nspheres > kFewSpheres, g.npoints > 32, fast_frame(fc)), grid, kTmemBlock,
+    return launch_overlapped(k_step_stream_tmem<true, false, 0, false>, grid, kTmemBlock, smem, st, g, fc);
+  return launch_overlapped(dftl_step_tmem(fc.nspheres > kFewSpheres, step_pairs(g, fc), fast_frame(fc)), grid, kTmemBlock,
                            smem, st, g, fc);
 }
 
@@ -440,17 +463,25 @@ int plain_mapping(const GroomView& g, const FrameConst& fc, int mapping) {
   const int K = lane_group(fc.mode, fc.substeps, fc.iterations);
   if (mapping == HS_MAPPING_LANES || K == 0) return mapping == HS_MAPPING_LANES ? HS_MAPPING_LANES : HS_MAPPING_THREAD;
   if (mapping == HS_MAPPING_THREAD) return HS_MAPPING_THREAD;
-  // AUTO: lane groups while a thread per strand leaves the SMs' schedulers
-  // short of warps and the lane groups do not crowd them. Measured on
-  // 1,024-65,536 strands x 16-64 points, 4 and 8 substeps: lane groups are
-  // faster up to about 16 of their warps per SM at 16 points, about N at
-  // N points (a longer chain gains more from the wavefront), slower beyond,
-  // where the idle lanes of the wavefront's head and tail and its shuffles
-  // cost more than the shorter chain saves.
+  // AUTO: lane groups while they make at most `limit` warps per SM (32-strand
+  // tiles x K). Their time grows with those warps times the wavefront's N + 2 S
+  // steps; a thread per strand takes S N chain links whatever the warps, until
+  // these fill the SMs. So the two meet at a multiple of S N / (N + 2 S), the
+  // larger the more sphere tests a thread runs in turn. Measured multiples
+  // (2 - 16 substeps, 4 - 64 points): 2.5 - 4 without spheres (5 up to 8
+  // points, where a thread per strand is the register form), 4.3 - 6.5 at one,
+  // 6.5 - 9.5 at 3 - 7, 7.2 - 13 at 10 - 32. Lanes / thread, us a frame (EXACT):
+  // 20,000 x 16, S 4, 7 spheres (16.4 warps) 8.2 / 11.0, 50,000 x 64 (41.1)
+  // 65.4 / 45.0, 54,476 x 32 without spheres (44.8) 31.0 / 17.4. A group of
+  // two holds few warps of long strands in shared memory, and gains only while
+  // they are resident together (22,431 x 64, S 2: 27.3 / 19.7).
+  const uint32_t N = g.npoints, S = static_cast<uint32_t>(fc.substeps);
+  const float multiple = fc.nspheres > 8 ? 8.5f : fc.nspheres > 1 ? 7.0f : fc.nspheres == 1 || N <= 8 ? 5.0f : 3.0f;
+  float limit = multiple * static_cast<float>(S * N) / static_cast<float>(N + 2 * S);
+  if (K == 2) limit = std::min(limit, 2.0f * static_cast<float>(227u / N));  // blocks of 1 KB a point
   const int sms = device_attribute(cudaDevAttrMultiProcessorCount, 152);
-  const uint64_t warps = static_cast<uint64_t>((g.nstrands + 31) / 32) * static_cast<uint64_t>(K);
-  const uint64_t per_sm = static_cast<uint64_t>(kLanesWarpsPerSm) * std::max<uint32_t>(16u, g.npoints) / 16u;
-  return warps <= per_sm * static_cast<uint64_t>(sms) ? HS_MAPPING_LANES : HS_MAPPING_THREAD;
+  const float warps = static_cast<float>((static_cast<uint64_t>(g.nstrands) + 31) / 32 * static_cast<uint64_t>(K));
+  return warps <= limit * static_cast<float>(sms) ? HS_MAPPING_LANES : HS_MAPPING_THREAD;
 }
 
 cudaError_t launch_step(const GroomView& g, const FrameConst& fc, int mapping, cudaStream_t st) {
