@@ -204,14 +204,14 @@ int step_pairs(const GroomView& g, const FrameConst& fc) {
   return fc.nspheres > 8 || g.npoints > 48 ? 2 : 0;
 }
 
-using TmemStep = void (*)(GroomView, FrameConst);
+using StepKernel = void (*)(GroomView, FrameConst);
 template <bool FAST>
-TmemStep dftl_step_tmem(bool many, int pairs) {
+StepKernel dftl_step_tmem(bool many, int pairs) {
   if (pairs == 2) return k_step_stream_tmem<false, false, 2, FAST>;
   if (pairs == 1) return k_step_stream_tmem<false, false, 1, FAST>;
   return many ? k_step_stream_tmem<false, true, 0, FAST> : k_step_stream_tmem<false, false, 0, FAST>;
 }
-TmemStep dftl_step_tmem(bool many, int pairs, bool fast) {
+StepKernel dftl_step_tmem(bool many, int pairs, bool fast) {
   return fast ? dftl_step_tmem<true>(many, pairs) : dftl_step_tmem<false>(many, pairs);
 }
 
@@ -235,8 +235,11 @@ cudaError_t launch_step_stream_tmem(const GroomView& g, const FrameConst& fc, cu
 
 // Lane groups (hs_lanes.cuh): a block of K warps per 32-strand tile, the
 // tile's starting state in shared memory ([npoints][32] positions, then
-// velocities). Register cap 128 (16 warps a SM).
-template <int K, bool FAST>
+// velocities). Register cap 128 (16 warps a SM). MANY: the push-out's form
+// for grooms among many spheres (push_seg), where a strand reaches a dozen of
+// them: us a frame without -> with, 8 substeps, EXACT, 2,858 x 41 among 18
+// 25.1 -> 15.7, 4,096 x 64 among 32 59 -> 39, 8,192 x 24 among 32 37 -> 35.
+template <int K, bool FAST, bool MANY>
 __global__ void __launch_bounds__(K * 32, 16 / K) k_step_lanes(GroomView g, FrameConst fc) {
   extern __shared__ float4 s_state[];
   __shared__ float4 s_c[HS_MAX_SPHERES];
@@ -246,22 +249,23 @@ __global__ void __launch_bounds__(K * 32, 16 / K) k_step_lanes(GroomView g, Fram
   frame_release();
   const SphereSet S = stage_spheres(fc, s_c, s_r2, s_adj);
   frame_acquire();
-  tile_frame_lanes<K, FAST>(fc, S, g, blockIdx.x, s_state, s_state + g.npoints * 32, s_ts);
+  tile_frame_lanes<K, FAST, MANY>(fc, S, g, blockIdx.x, s_state, s_state + g.npoints * 32, s_ts);
 }
 
 template <int K>
 cudaError_t launch_step_lanes_k(const GroomView& g, const FrameConst& fc, cudaStream_t st) {
   const unsigned grid = (g.nstrands + 31) / 32;
   const size_t smem = 2 * sizeof(float4) * 32 * g.npoints;
+  static const StepKernel kernels[2][2] = {{k_step_lanes<K, false, false>, k_step_lanes<K, false, true>},
+                                         {k_step_lanes<K, true, false>, k_step_lanes<K, true, true>}};
   static std::atomic<uint64_t> optin{0};
   once_per_device(optin, [] {
     const int bytes = 2 * static_cast<int>(sizeof(float4)) * 32 * HS_MAX_POINTS_PER_STRAND;
-    cudaFuncSetAttribute(k_step_lanes<K, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    cudaFuncSetAttribute(k_step_lanes<K, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    for (const auto& contract : kernels)
+      for (const StepKernel k : contract) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
   });
-  const unsigned block = K * 32;
-  if (fast_frame(fc)) return launch_overlapped(k_step_lanes<K, true>, grid, block, smem, st, g, fc);
-  return launch_overlapped(k_step_lanes<K, false>, grid, block, smem, st, g, fc);
+  const StepKernel k = kernels[fast_frame(fc) ? 1 : 0][fc.nspheres > kFewSpheres ? 1 : 0];
+  return launch_overlapped(k, grid, K * 32, smem, st, g, fc);
 }
 
 cudaError_t launch_step_lanes(const GroomView& g, const FrameConst& fc, cudaStream_t st) {

@@ -59,7 +59,8 @@ __device__ __forceinline__ void load_start(bool take, const float4* sp, const fl
 // the strand's starting segments (point 0: its world position) with the
 // rest lengths in w, s_v its velocities, [point][32] at column c. The lane
 // of the last substep stores the finished points and adds them to `ts`.
-template <int K, bool FAST, int NF>
+// MANY: the push-out's form for grooms among many spheres (push_seg).
+template <int K, bool FAST, bool MANY, int NF>
 __device__ __forceinline__ void lanes_pass(const FrameConst& fc, const StrandConsts& Kc, const SphereFilter<NF>& F,
                                            const SphereSet& S, const GroomView& g, uint32_t s, bool active, int c,
                                            int k, int n, int jmin, V3 x0_start, V3 target, float rest0,
@@ -109,7 +110,7 @@ __device__ __forceinline__ void lanes_pass(const FrameConst& fc, const StrandCon
     const V3 w_i = add(w_prev, sn);
     // Finish point j - 1 (2 <= j <= n).
     const bool fin = worker && j >= 2 && j <= n;
-    if (fin && j - 1 >= jmin && flagged(F, w_prev)) push_seg<false, FAST>(F, S, w_prev, D_prev, s_prev, sn, tip);
+    if (fin && j - 1 >= jmin && flagged(F, w_prev)) push_seg<MANY, FAST>(F, S, w_prev, D_prev, s_prev, sn, tip);
     const V3 vel = vel_of(Kc, tip ? D_prev : fmas(Kc.neg_damping, e, D_prev));
     if (writer && fin) {
       wout = add(wout, s_prev);
@@ -151,7 +152,7 @@ __device__ __forceinline__ void lanes_pass(const FrameConst& fc, const StrandCon
 // warp w takes strands [w 32/K, (w + 1) 32/K) of the tile, lane l strand
 // l / K as substep lane l % K). s_p, s_v: [n][32] float4 each, the tile's
 // starting state; s_ts: 32 TileStats. Every thread of the block calls it.
-template <int K, bool FAST>
+template <int K, bool FAST, bool MANY = false>
 __device__ __forceinline__ void tile_frame_lanes(const FrameConst& fc, const SphereSet& S, const GroomView& g,
                                                  uint32_t tile, float4* s_p, float4* s_v, TileStats* s_ts) {
   static_assert(K == 2 || K == 4 || K == 8 || K == 16, "lane groups of 2, 4, 8 or 16");
@@ -223,7 +224,7 @@ __device__ __forceinline__ void tile_frame_lanes(const FrameConst& fc, const Sph
   const SphereFilter<8> F = filter_spheres<8>(S, reach, far);
   TileStats ts;
   ts.init();
-  lanes_pass<K, FAST>(fc, Kc, F, S, g, s, active, c, k, n, jmin, x0_start, target, rest0, s_p, s_v, ts);
+  lanes_pass<K, FAST, MANY>(fc, Kc, F, S, g, s, active, c, k, n, jmin, x0_start, target, rest0, s_p, s_v, ts);
 
   // Tile statistics: the strands' own (from their last substep's lane, in
   // point order), reduced by one warp as the thread-per-strand kernels do.

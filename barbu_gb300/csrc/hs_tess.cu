@@ -7,9 +7,9 @@
 // tangents from the groom's [point][strand] arrays) and the line's triangle
 // sample once, evaluates the tessellation evaluation shader at each of the
 // line's nsub + 1 vertices, and writes the line's 2 nsub segment ends into
-// shared memory; the warp then stores its 32 lines, which are contiguous in
-// the output, with coalesced writes. The shader's divisions, the Hermite
-// basis at each u and the smoothstep of each (point, u) pair come from
+// shared memory, from where the copy engine takes them to the output as one
+// bulk copy. The shader's divisions, the Hermite basis at each u, the
+// smoothstep of each (point, u) pair and the triangle samples come from
 // per-block tables (one entry per distinct operand).
 //
 // Arithmetic contract (shared with the oracle, which matches bit for bit):
