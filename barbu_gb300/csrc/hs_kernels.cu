@@ -185,7 +185,8 @@ constexpr int kFewSpheres = 8;
 // less):
 //   less than a wave  60,000 x 32 among 7 spheres 48.5 / 42.8, among 32 126 /
 //                     93; 60,000 x 16 among 24 48.9 / 42.0; 50,021 x 12 among
-//                     7 16.5 / 17.2; 38,133 x 32 without 10.8 / 11.9 (S 4);
+//                     7 16.5 / 17.2, x 23 with two exports (S 5) 37.3 / 37.8;
+//                     38,133 x 32 without 10.8 / 11.9 (S 4);
 //                     20,000 x 36 among 8 47.7 / 35.5 / 36.6
 //   more              262,144 x 32 among 7 125 / 131; 150,000 x 36 among 4 111
 //                     / 113 / 117; 150,000 x 64 among 4 180 / 175 / 172, among
@@ -198,7 +199,7 @@ int step_pairs(const GroomView& g, const FrameConst& fc) {
   const bool is_long = g.npoints > 32;
   const uint32_t sms = static_cast<uint32_t>(device_attribute(cudaDevAttrMultiProcessorCount, 152));
   const bool wave = (g.nstrands + 31) / 32 <= (is_long ? 8u : 16u) * sms;
-  if (!is_long) return wave && fc.nspheres > 1 && (g.npoints > 20 || fc.nspheres > 16) ? 1 : 0;
+  if (!is_long) return wave && fc.nspheres > 1 && (g.npoints > 24 || fc.nspheres > 16) ? 1 : 0;
   if (fc.nspheres == 0) return g.npoints > 48 ? 2 : 0;
   if (fc.nspheres == 1 || wave) return 1;
   return fc.nspheres > 8 || g.npoints > 48 ? 2 : 0;
