@@ -493,16 +493,19 @@ static cudaError_t ensure_capacity(hs_ctx* ctx, BatchState& B, uint32_t n) {
   return e;
 }
 
-// A groom set's shape: grooms, modes, point counts, and what decides
-// whether a bucket can take lane groups (substeps, iterations).
+// What the plan of a groom set follows from: each groom's strands, points,
+// mode and contract, and what decides whether a bucket can take lane groups
+// (substeps, iterations: at most 64 each). A groom's address alone does not
+// tell it from one that was destroyed.
 static std::vector<uint64_t> signature_of(hs_groom* const* grooms, uint32_t n) {
   std::vector<uint64_t> sig;
-  sig.reserve(3 * n);
+  sig.reserve(3 * static_cast<size_t>(n));
   for (uint32_t i = 0; i < n; ++i) {
-    sig.push_back(reinterpret_cast<uint64_t>(grooms[i]));
-    sig.push_back((static_cast<uint64_t>(grooms[i]->sim.mode) << 32) | grooms[i]->npoints);
-    sig.push_back((static_cast<uint64_t>(grooms[i]->sim.substeps) << 32) |
-                  (static_cast<uint64_t>(grooms[i]->sim.iterations) << 8) | grooms[i]->sim.contract);
+    const hs_groom& g = *grooms[i];
+    sig.push_back(reinterpret_cast<uint64_t>(&g));
+    sig.push_back((static_cast<uint64_t>(g.nstrands) << 32) | g.npoints);
+    sig.push_back((static_cast<uint64_t>(g.sim.substeps) << 32) | (static_cast<uint64_t>(g.sim.iterations) << 16) |
+                  (static_cast<uint64_t>(g.sim.mode) << 8) | g.sim.contract);
   }
   return sig;
 }
