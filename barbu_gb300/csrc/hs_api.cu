@@ -111,14 +111,11 @@ hs_status make_frame_const(const hs_groom* g, float dt, FrameConst* out) {
   fc.nspheres = static_cast<int32_t>(g->spheres.size());
   fc.wind_key = stream_key(g->seed, kStreamWind);
   fc.contract = static_cast<int32_t>(p.contract);
-  float rmax = 0.0f;
   const size_t K = g->spheres.size();
   for (size_t k = 0; k < K; ++k) {
     fc.spheres[k] = g->spheres[k];
     fc.r2[k] = g->spheres[k].w * g->spheres[k].w;
-    rmax = std::fmax(rmax, g->spheres[k].w);
   }
-  fc.sphere_rmax = rmax;
   std::memcpy(fc.adj, g->adj, sizeof(fc.adj));
   std::memcpy(fc.bone_real, g->bone_real, sizeof(fc.bone_real));
   std::memcpy(fc.bone_dual, g->bone_dual, sizeof(fc.bone_dual));

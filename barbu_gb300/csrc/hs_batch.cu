@@ -152,9 +152,9 @@ __global__ void __maxnreg__(128)
 // memory holds the table entries and the positions, 12 bytes a point.
 // WARPS (4 or 8) is compile-time, so the shared-memory strides are
 // immediates; resident blocks are bounded by TMEM and shared memory at 16
-// warps per SM (8 for more than 32 points), and registers with them. P:
-// pairs of substeps at once (WavePass): none, or 1 for a bucket of less than
-// a wave of warps, 2 for more than 32 points.
+// warps per SM (8 for more than 32 points), and registers with them. P: the
+// most pairs of substeps its grooms may run at once (FrameConst::pairs,
+// WavePass): none, 1, or 2 for more than 32 points.
 template <bool REF, int WARPS, bool FAST, int P>
 __global__ void __launch_bounds__(WARPS * 32, (P == 2 ? 8 : 16) / WARPS)
     k_step_batch_stream_tmem(const BucketHeader* __restrict__ hdr, const BucketDir* __restrict__ dirs,
@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(WARPS * 32, (P == 2 ? 8 : 16) / WARPS)
     }
     const uint32_t s = strand0 + lane;
     const SphereSet S{e.fc.spheres, e.fc.r2, e.fc.adj, e.fc.nspheres};
-    strand_frame_stream<REF, XShared3, VTmem, kCachedSpheres, false, false, FAST, P, P == 1 ? 4 : 8>(
+    strand_frame_stream<REF, XShared3, VTmem, kCachedSpheres, false, false, FAST, P, P == 1 ? 4 : 8, P != 0>(
         e.fc, S, e.view, s, s < e.view.nstrands, X, V);
   }
   tmem::fence_before_sync();
@@ -251,7 +251,7 @@ const void* tmem_kernel(int warps) {
   return nullptr;
 }
 
-// pairs: pairs of substeps at once (tensor-memory DFTL kernels).
+// pairs: Bucket::pairs (tensor-memory DFTL kernels).
 template <bool REF, bool FAST>
 const void* any_cap_kernel(int variant, int warps, int pairs) {
   if (is_lanes(variant)) {
@@ -374,18 +374,54 @@ cudaKernelNodeParams node_params(const Bucket& bk, LaunchArgs* a) {
 
 }  // namespace
 
-// Pairs of substeps a bucket of `ntiles` 32-strand tiles runs at once: two
-// for more than 32 points (8 warps an SM), one where its tiles are no more
-// than the 16 warps an SM holds (48 grooms of 256 - 4,096 strands, 2,054
-// tiles on 2,432 warps: 48 - 58 -> 40 - 42 us a frame; 4,155 tiles of such
-// grooms: 63 -> 72 us, where the GPU is busy with other work too), else
-// none. (The occupancy query answers one block an SM for kernels that
-// allocate tensor memory, so it does not say how many warps there are.)
-static int substep_pairs(int cap, int cls, int variant, uint32_t ntiles) {
-  if (!is_tmem(variant) || cls == kClassRef) return 0;
+// The most pairs of substeps the grooms of a bucket may run at once: two for
+// more than 32 points, where tensor memory leaves an SM 8 warps and the
+// registers for them; one for a bucket of at most the 16 warps an SM holds;
+// above that schedulers are busy (4,155 tiles of 8 - 32 points: 63 us with
+// none, 72 with one). (The occupancy query answers one block an SM for
+// kernels that allocate tensor memory, so it does not say how many warps
+// there are.)
+static int most_pairs(int cap, int cls, uint32_t ntiles) {
+  if (cls == kClassRef) return 0;
   if (cap > 32) return 2;
-  const int sms = device_attribute(cudaDevAttrMultiProcessorCount, 152);
-  return ntiles <= 16u * static_cast<uint32_t>(sms) ? 1 : 0;
+  const uint32_t sms = static_cast<uint32_t>(device_attribute(cudaDevAttrMultiProcessorCount, 152));
+  return ntiles <= 16u * sms ? 1 : 0;
+}
+
+// Pairs of substeps of the grooms of a bucket that may run `most`, chosen anew
+// each frame: a set's spheres may change without a new plan. They pay where a
+// warp waits on chain links and its sphere tests run two-wide, and cost the
+// steps between sweeps and an odd substep's change of form.
+//
+// Up to 32 points: all grooms or none, as the slowest tile gains (`points`,
+// `spheres`: its). Its warp is the frame's length, and warps in the two forms
+// at once evict each other's instructions (48 grooms among 1 - 16 spheres,
+// each by itself: 47 us where all in pairs take 40). us a frame, one substep
+// at a time / pairs (update_many, EXACT; 8 substeps unless S is given; 48
+// grooms of 256 - 4,096 strands unless said):
+//   no sphere 31.1 / 34.3, one (S 5) 35.9 / 47.0; 16 113.9 / 78.2, 32 (S 5)
+//   159.6 / 103.9; 1 - 16 each 147.9 / 99.6, S 5 99.6 / 79.6; 1 - 4 each 63.1 /
+//   63.0, S 5 48.6 / 53.4; x 24 among 12 77.8 / 71.3, S 5 64.1 / 64.1; x 32
+//   among 4 71.4 / 66.5; x 12 among 12 39.4 / 37.4, x 10 37.1 / 40.9
+//   less than a warp a scheduler: 16 grooms of 200 - 600 x 16 - 32, one sphere
+//   29.6 / 27.8
+// More: each groom by itself. One pair beside two where both were timed.
+//   64 grooms of 300 - 1,000 x 40 (less than the 8 warps an SM) among 4 68.7 /
+//   64.7, among 16 (S 5) 105.0 / 82.4; of 1,000 - 4,000 among 8 228 / 208 (two
+//   299), S 5 169.5 / 180.5, among 32 (S 5) 692.8 / 465.6, one sphere (S 2)
+//   117.0 / 119.3; x 64 without spheres (FAST) 206 / 196 (two 180)
+static int bucket_pairs(const FrameConst& fc, uint32_t points, uint32_t spheres, int most, uint32_t ntiles,
+                        uint32_t sms) {
+  if (most == 0 || fc.mode != HS_MODE_DFTL || fc.iterations != 1 || fc.substeps < 2) return 0;
+  const bool even = fc.substeps % 2 == 0;
+  if (most == 2) {
+    if (spheres == 0 && points > 48) return 2;
+    return ntiles <= 8u * sms || spheres > 16 || (even && (fc.substeps > 2 || spheres > 8)) ? 1 : 0;
+  }
+  if (spheres > 24) return 1;
+  if (points <= 12) return even && points == 12 && spheres > 10 ? 1 : 0;
+  if (!even) return spheres > 12 ? 1 : 0;
+  return spheres > (ntiles <= 4u * sms ? 0u : 3u) ? 1 : 0;
 }
 
 int batch_occupancy(int cap, int cls, int variant, int warps_per_block, int pairs) {
@@ -528,6 +564,13 @@ static bool shape_fits(const Bucket& bk, const TuneChoice& c) {
   return !is_lanes(c.variant) || (bk.lanes_k > 0 && c.warps_per_block >= bk.lanes_k);
 }
 
+// The kernel of a bucket: the most pairs of substeps it runs, and its grid.
+static void set_kernel(Bucket* bk, int sms, int pairs) {
+  bk->pairs = pairs;
+  const int occ = std::max(1, batch_occupancy(bk->cap, bk->cls, bk->variant, bk->warps_per_block, pairs));
+  bk->grid = static_cast<uint32_t>(sms * occ * bk->waves);
+}
+
 // Groups a new groom set into buckets with their directories and shapes.
 static void regroup(hs_ctx* ctx, BatchState& B, hs_groom* const* grooms, uint32_t n) {
   // One flat work list: every DFTL groom of up to 32 points shares one
@@ -561,6 +604,8 @@ static void regroup(hs_ctx* ctx, BatchState& B, hs_groom* const* grooms, uint32_
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
   B.buckets.clear();
   B.dirs.clear();
+  B.bucket_of.assign(n, 0);
+  B.sms = sms;
   B.headers.assign(kMaxBuckets, BucketHeader{0, 0, 0, 0});
   // Longest tiles first, so that the frame ends on the shortest ones and
   // its last partial wave is short: buckets launch in descending point
@@ -594,9 +639,10 @@ static void regroup(hs_ctx* ctx, BatchState& B, hs_groom* const* grooms, uint32_
     if (!shape_fits(bk, tc)) tc = default_choice(bk.cap);
     bk.variant = tc.variant;
     bk.warps_per_block = tc.warps_per_block;
-    bk.pairs = substep_pairs(bk.cap, bk.cls, bk.variant, tiles);
-    const int occ = std::max(1, batch_occupancy(bk.cap, bk.cls, bk.variant, bk.warps_per_block, bk.pairs));
-    bk.grid = static_cast<uint32_t>(sms * occ * tc.waves);
+    bk.waves = tc.waves;
+    bk.most_pairs = most_pairs(bk.cap, bk.cls, tiles);
+    set_kernel(&bk, sms, bk.most_pairs == 1 && !B.pairs_ran ? 0 : bk.most_pairs);
+    for (uint32_t i : kv.second) B.bucket_of[i] = static_cast<uint32_t>(B.buckets.size());
     // Bucket b of the launch reads header and counter slot b.
     B.headers[B.buckets.size()] = h;
     B.buckets.push_back(bk);
@@ -605,16 +651,38 @@ static void regroup(hs_ctx* ctx, BatchState& B, hs_groom* const* grooms, uint32_
   B.ngrooms = n;
 }
 
-// Fills a staging slot: headers, directory, table.
+// Fills a staging slot: headers, directory, table. A bucket whose grooms run
+// pairs of substeps for the first time takes the kernel that has them, and
+// keeps it (one more graph): that kernel runs grooms without pairs as fast but
+// for FAST ones without spheres (48 grooms, 8 substeps: 29.7 us against 32.2).
 static hs_status fill(BatchState& B, int slot, hs_groom* const* grooms, uint32_t n, float dt) {
   char* h = B.h_buf[slot];
   std::memcpy(h, B.headers.data(), sizeof(BucketHeader) * kMaxBuckets);
   std::memcpy(h + B.dir_offset(), B.dirs.data(), sizeof(BucketDir) * B.dirs.size());
   BatchGroomDev* table = reinterpret_cast<BatchGroomDev*>(h + B.table_offset());
+  uint32_t slowest[kMaxBuckets], cost[kMaxBuckets] = {0};  // the groom of each bucket whose tiles take longest
   for (uint32_t i = 0; i < n; ++i) {
     hs_status st = make_frame_const(grooms[i], dt, &table[i].fc);
     if (st != HS_OK) return st;
     table[i].view = view_of(grooms[i]);
+    // Chain links and, per sphere, about a quarter of one.
+    const uint32_t b = B.bucket_of[i], c = grooms[i]->npoints * (4u + static_cast<uint32_t>(table[i].fc.nspheres));
+    if (c > cost[b]) {
+      cost[b] = c;
+      slowest[b] = i;
+    }
+  }
+  for (uint32_t i = 0; i < n; ++i) {
+    Bucket& bk = B.buckets[B.bucket_of[i]];
+    if (bk.most_pairs == 0) continue;
+    const BatchGroomDev& by = table[bk.most_pairs == 2 ? i : slowest[B.bucket_of[i]]];
+    const int pairs = bucket_pairs(table[i].fc, by.view.npoints, static_cast<uint32_t>(by.fc.nspheres), bk.most_pairs,
+                                   bk.ntiles, static_cast<uint32_t>(B.sms));
+    table[i].fc.pairs = pairs;
+    if (pairs > bk.pairs) {
+      B.pairs_ran = true;
+      set_kernel(&bk, B.sms, bk.most_pairs);
+    }
   }
   return HS_OK;
 }
@@ -776,8 +844,7 @@ static hs_status autotune(hs_ctx* ctx, hs_groom* const* grooms, uint32_t n, floa
         Bucket trial = bk;
         trial.variant = variant;
         trial.warps_per_block = wpb;
-        trial.pairs = substep_pairs(bk.cap, bk.cls, variant, bk.ntiles);
-        const int occ = batch_occupancy(bk.cap, bk.cls, variant, wpb, trial.pairs);
+        const int occ = batch_occupancy(bk.cap, bk.cls, variant, wpb, bk.pairs);
         if (occ <= 0) continue;
         for (int waves : {1, 2, 4}) {
           trial.grid = static_cast<uint32_t>(sms * occ * waves);
@@ -878,7 +945,7 @@ HS_API hs_status hs_tune_override(hs_ctx* ctx, uint32_t points, uint32_t mode, u
   if (waves != 1 && waves != 2 && waves != 4) return fail(HS_ERR_INVALID_ARG, "hs_tune_override: waves must be 1, 2 or 4");
   const int cls = mode == HS_MODE_REFERENCE ? kClassRef : kClassExact;
   if (batch_occupancy(cap, cls, static_cast<int>(variant), static_cast<int>(warps_per_block),
-                      substep_pairs(cap, cls, static_cast<int>(variant), 1)) <= 0)
+                      most_pairs(cap, cls, 1)) <= 0)
     return fail(HS_ERR_UNSUPPORTED, "hs_tune_override: that shape does not fit on an SM");
   if (!ctx->tune) ctx->tune = new TuneCache();
   ctx->tune->pinned[std::make_pair(cap, mode == HS_MODE_REFERENCE)] =

@@ -75,7 +75,9 @@ struct Bucket {
   int cls = kClassExact;  // step class
   int variant = kVariantRegs;
   int warps_per_block = 4;
-  int pairs = 0;  // pairs of substeps the kernel runs at once (substep_pairs)
+  int most_pairs = 0;  // pairs of substeps its grooms may run at once
+  int pairs = 0;       // those of its present tensor-memory kernel (0: not yet asked for)
+  int waves = 1;       // TuneChoice::waves
   uint32_t grid = 1;
   uint32_t ntiles = 0;
   int lanes_k = 0;  // smallest lane group every groom of the bucket fits (0: none, lane_group)
@@ -95,6 +97,9 @@ struct BatchState {
   uint32_t ngrooms = 0;
   std::vector<Bucket> buckets;          // bucket b uses header/counter slot b
   std::vector<BucketDir> dirs;          // grouped by bucket
+  std::vector<uint32_t> bucket_of;      // the bucket of each groom
+  bool pairs_ran = false;               // a bucket of up to 32 points has run pairs of substeps
+  int sms = 0;                          // of the context's device
   std::vector<BucketHeader> headers;
   // The frame graph: counter reset, table copy, one kernel per bucket.
   cudaGraph_t graph = nullptr;
@@ -128,7 +133,7 @@ struct TuneCache {
 TuneKey tune_key(int cap, int cls, uint32_t ntiles);
 TuneChoice tuned_choice(hs_ctx* ctx, int cap, int cls, uint32_t ntiles);
 TuneChoice default_choice(int cap);  // the untuned shape of a capacity
-// pairs: pairs of substeps at once (Bucket::pairs).
+// pairs: Bucket::pairs.
 int batch_occupancy(int cap, int cls, int variant, int warps_per_block, int pairs);
 hs_status batch_update(hs_ctx* ctx, hs_groom* const* grooms, uint32_t n, float dt);
 

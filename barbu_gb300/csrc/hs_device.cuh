@@ -202,7 +202,7 @@ struct FrameConst {
   int32_t substeps, iterations, mode, root_mode;
   int32_t nspheres;
   uint32_t wind_key;
-  float sphere_rmax;        // largest sphere radius (culling bound)
+  int32_t pairs;            // pairs of substeps at once in a bucket's kernel (bucket_pairs)
   int32_t contract;         // hs_contract of the DFTL chain link
   float4 spheres[HS_MAX_SPHERES];  // (x, y, z, r)
   float r2[HS_MAX_SPHERES];        // r * r

@@ -1071,10 +1071,10 @@ struct WavePass {
 // (an odd last one, short strands) go one at a time (substeps_seg).
 template <int P, bool FAST, typename XS, typename VS, int NF>
 __device__ __forceinline__ int wave_substeps(const FrameConst& fc, const StrandConsts& K, const SphereFilter<NF>& F1,
-                                             const SphereSet& S, int n, int jmin, const XS& X, const VS& V) {
+                                             const SphereSet& S, int n, int jmin, int pairs, const XS& X, const VS& V) {
   const SphereFilter2<NF> F(F1);
   int k = 0;
-  if (P > 1 && n >= kWaveMinPoints<2 * P> && fc.substeps >= 2 * P) {
+  if (P > 1 && pairs >= P && n >= kWaveMinPoints<2 * P> && fc.substeps >= 2 * P) {
     WavePass<P, FAST, XS, VS, NF> pass{K, fc, F, S, X, V, n, jmin, 0, negative_zero()};
     pass.run(fc.substeps / (2 * P));
     k = fc.substeps / (2 * P) * (2 * P);
@@ -1159,12 +1159,11 @@ __device__ __forceinline__ void substeps_ref(const FrameConst& fc, const StrandC
   }
 }
 
-// Substeps k0 .. substeps - 1, one at a time, then the root's slot.
+// Substeps k0 .. substeps - 1, one at a time.
 template <bool SPLIT, bool PICK, bool FAST, typename XS, typename VS, int NF>
 __device__ __forceinline__ void substeps_seg(const FrameConst& fc, const StrandConsts& K, const SphereFilter<NF>& F,
-                                             const SphereSet& S, int n, int jmin, int k0, V3 x0_start, V3 target,
-                                             float rest0, const XS& X, const VS& V) {
-  const RootPath path{x0_start, target, fc.substeps, fc.root_mode != HS_ROOT_PINNED};
+                                             const SphereSet& S, int n, int jmin, int k0, const RootPath& path,
+                                             const XS& X, const VS& V) {
   V3 rel_prev = path.rel(k0 - 1);
   for (int k = k0; k < fc.substeps; ++k) {
     const V3 rel = path.rel(k), D0 = sub(rel, rel_prev), R = path.at(k, rel);
@@ -1175,10 +1174,6 @@ __device__ __forceinline__ void substeps_seg(const FrameConst& fc, const StrandC
     }
     V.fence();
   }
-  const V3 D0 = sub(path.rel(fc.substeps - 1), path.rel(fc.substeps - 2));
-  X.store(0, f4(v3(0.0f, 0.0f, 0.0f), rest0));
-  V.store(0, f4(vel_of(K, D0), vel_w<XS>(rest0)));
-  V.fence();
 }
 
 // One frame of strand s. X: the position/segment slots (XShared4 or
@@ -1193,8 +1188,10 @@ __device__ __forceinline__ void substeps_seg(const FrameConst& fc, const StrandC
 // loop; the plain step splits it.
 // PICK: the push-out's form (push_seg). P: pairs of substeps at once
 // (WavePass; 0: one substep at a time). NF: slots of the sphere filter.
+// EACH: grooms of fewer pairs share the kernel (FrameConst::pairs); those of
+// none test 8 slots, whatever NF.
 template <bool REF, typename XS, typename VS, int M = kCachedSpheres, bool SPLIT = false, bool PICK = false,
-          bool FAST = false, int P = 0, int NF = 8>
+          bool FAST = false, int P = 0, int NF = 8, bool EACH = false>
 __device__ __forceinline__ void strand_frame_stream(const FrameConst& fc, const SphereSet& S, const GroomView& g,
                                                     uint32_t s, bool active, const XS& X, const VS& V) {
   const int n = static_cast<int>(g.npoints);
@@ -1283,20 +1280,33 @@ __device__ __forceinline__ void strand_frame_stream(const FrameConst& fc, const 
         jmin = __reduce_min_sync(0xffffffffu, active ? jl : n);
       }
     }
-    const SphereFilter<NF> F = filter_spheres<NF>(S, reach, far);
-    int k0 = 0;  // substeps done in pairs
-    if constexpr (P > 0) {
-      // The root's path waits in slot 0.
-      X.store(0, f4(x0_start, rest0));
-      V.store(0, f4(target, rest0));
-      if (fc.iterations == 1) k0 = wave_substeps<P, FAST>(fc, K, F, S, n, jmin, X, V);
-      V.fence();
-      const float4 v0 = V.load(0);
-      x0_start = xyz(X.load(0));
-      target = xyz(v0);
-      rest0 = v0.w;
+    const bool moves = fc.root_mode != HS_ROOT_PINNED;
+    if (EACH && NF != 8 && fc.pairs == 0) {
+      substeps_seg<SPLIT, PICK, FAST>(fc, K, filter_spheres<8>(S, reach, far), S, n, jmin, 0,
+                                      RootPath{x0_start, target, fc.substeps, moves}, X, V);
+    } else {
+      const SphereFilter<NF> F = filter_spheres<NF>(S, reach, far);
+      int k0 = 0;  // substeps done in pairs
+      if constexpr (P > 0) {
+        if (!EACH || fc.pairs > 0) {
+          // The root's path waits in slot 0.
+          X.store(0, f4(x0_start, rest0));
+          V.store(0, f4(target, rest0));
+          k0 = wave_substeps<P, FAST>(fc, K, F, S, n, jmin, EACH ? fc.pairs : P, X, V);
+          V.fence();
+          const float4 v0 = V.load(0);
+          x0_start = xyz(X.load(0));
+          target = xyz(v0);
+          rest0 = v0.w;
+        }
+      }
+      substeps_seg<SPLIT, PICK, FAST>(fc, K, F, S, n, jmin, k0, RootPath{x0_start, target, fc.substeps, moves}, X, V);
     }
-    substeps_seg<SPLIT, PICK, FAST>(fc, K, F, S, n, jmin, k0, x0_start, target, rest0, X, V);
+    const RootPath path{x0_start, target, fc.substeps, moves};
+    const V3 D0 = sub(path.rel(fc.substeps - 1), path.rel(fc.substeps - 2));
+    X.store(0, f4(v3(0.0f, 0.0f, 0.0f), rest0));
+    V.store(0, f4(vel_of(K, D0), vel_w<XS>(rest0)));
+    V.fence();
   }
 
   // Store: reference mode holds positions; DFTL mode rebuilds them from the
