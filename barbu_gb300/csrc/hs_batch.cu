@@ -769,7 +769,7 @@ hs_status batch_update(hs_ctx* ctx, hs_groom* const* grooms, uint32_t n, float d
 TuneKey tune_key(int cap, int cls, uint32_t ntiles) {
   int lg = 0;
   while (lg < 31 && (1u << (lg + 1)) <= ntiles) ++lg;
-  return TuneKey{cap, cls, lg};
+  return TuneKey{cap, cls, lg, most_pairs(cap, cls, ntiles)};
 }
 
 // Pins (hs_tune_override) are per (capacity, mode): both contracts of a
@@ -944,9 +944,11 @@ HS_API hs_status hs_tune_override(hs_ctx* ctx, uint32_t points, uint32_t mode, u
     return fail(HS_ERR_UNSUPPORTED, "hs_tune_override: lane groups run DFTL mode only");
   if (waves != 1 && waves != 2 && waves != 4) return fail(HS_ERR_INVALID_ARG, "hs_tune_override: waves must be 1, 2 or 4");
   const int cls = mode == HS_MODE_REFERENCE ? kClassRef : kClassExact;
-  if (batch_occupancy(cap, cls, static_cast<int>(variant), static_cast<int>(warps_per_block),
-                      most_pairs(cap, cls, 1)) <= 0)
-    return fail(HS_ERR_UNSUPPORTED, "hs_tune_override: that shape does not fit on an SM");
+  // In each form the bucket's kernel may take (set_kernel).
+  const int most = most_pairs(cap, cls, 1);
+  for (int pairs = most == 2 ? 2 : 0; pairs <= most; ++pairs)
+    if (batch_occupancy(cap, cls, static_cast<int>(variant), static_cast<int>(warps_per_block), pairs) <= 0)
+      return fail(HS_ERR_UNSUPPORTED, "hs_tune_override: that shape does not fit on an SM");
   if (!ctx->tune) ctx->tune = new TuneCache();
   ctx->tune->pinned[std::make_pair(cap, mode == HS_MODE_REFERENCE)] =
       TuneChoice{static_cast<int>(warps_per_block), static_cast<int>(waves), static_cast<int>(variant)};

@@ -121,8 +121,10 @@ struct TuneChoice {
   int variant = kVariantRegs;
 };
 
-// Key: (capacity, step class, log2 of the bucket's tile count).
-using TuneKey = std::tuple<int, int, int>;
+// Key: (capacity, step class, log2 of the bucket's tile count, most pairs of
+// substeps). The line at which buckets stop running pairs lies inside a power
+// of two of tiles: a shape timed on one side says nothing about the other.
+using TuneKey = std::tuple<int, int, int, int>;
 
 struct TuneCache {
   std::map<TuneKey, TuneChoice> best;

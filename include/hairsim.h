@@ -336,7 +336,9 @@ typedef struct hs_tune_entry {
   uint32_t contract;        /* hs_contract of the bucket's grooms (DFTL; each contract has its own kernels) */
 } hs_tune_entry;
 /* Copies up to `capacity` entries of the context's autotuner cache;
- * *out_count is the number of entries in the cache. */
+ * *out_count is the number of entries in the cache. A size class may have two
+ * entries, of buckets that fill the GPU and of smaller ones (the two run
+ * different kernels). */
 HS_API hs_status hs_tune_entries(hs_ctx* ctx, hs_tune_entry* out, uint32_t capacity, uint32_t* out_count);
 
 /* ---- serving ------------------------------------------------------------ */
