@@ -205,7 +205,10 @@ __global__ void __launch_bounds__(WARPS * 32, (P == 2 ? 8 : 16) / WARPS)
 // Lane groups (hs_lanes.cuh): a block of K warps takes one 32-strand tile
 // at a time from the bucket's counter. Shared memory: the groom's table
 // entry, then the tile's starting state ([cap][32] positions, then
-// velocities). Register cap 128 (16 warps a SM).
+// velocities). Register cap 128 (16 warps a SM). A groom among many spheres
+// takes the push-out's form for them, as in k_step_lanes: one groom of 4,096 x
+// 64 among 32, 8 substeps, EXACT, 62 -> 50 us; 48 grooms of 256 - 4,096 x 16
+// among 32 242 -> 187, among 4 85 (FAST 79 -> 80).
 template <int K, bool FAST>
 __global__ void __launch_bounds__(K * 32, 16 / K)
     k_step_batch_lanes(const BucketHeader* __restrict__ hdr, const BucketDir* __restrict__ dirs,
@@ -239,7 +242,10 @@ __global__ void __launch_bounds__(K * 32, 16 / K)
       __syncthreads();
     }
     const SphereSet S{e.fc.spheres, e.fc.r2, e.fc.adj, e.fc.nspheres};
-    tile_frame_lanes<K, FAST>(e.fc, S, e.view, strand0 / kWarp, s_p, s_v, s_ts);
+    if (e.fc.nspheres > kFewSpheres)
+      tile_frame_lanes<K, FAST, true>(e.fc, S, e.view, strand0 / kWarp, s_p, s_v, s_ts);
+    else
+      tile_frame_lanes<K, FAST, false>(e.fc, S, e.view, strand0 / kWarp, s_p, s_v, s_ts);
     __syncthreads();  // the next tile rewrites s_next, the entry and the state
   }
 }

@@ -174,10 +174,6 @@ size_t tmem_step_smem(uint32_t npoints) {
   return std::max(need, per_block > fixed ? per_block - fixed : need);
 }
 
-// Spheres of a groom up to which its strands reach few of them, and the
-// push-out goes through all of those (measured at 7 and 16: push_seg).
-constexpr int kFewSpheres = 8;
-
 // Pairs of substeps a DFTL groom runs at once. They pay where schedulers wait
 // on chain links: less than a wave of warps (16 an SM, 8 for more than 32
 // points), longer strands, sphere tests to run two-wide. Single pass against

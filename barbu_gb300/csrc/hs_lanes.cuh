@@ -152,7 +152,7 @@ __device__ __forceinline__ void lanes_pass(const FrameConst& fc, const StrandCon
 // warp w takes strands [w 32/K, (w + 1) 32/K) of the tile, lane l strand
 // l / K as substep lane l % K). s_p, s_v: [n][32] float4 each, the tile's
 // starting state; s_ts: 32 TileStats. Every thread of the block calls it.
-template <int K, bool FAST, bool MANY = false>
+template <int K, bool FAST, bool MANY>
 __device__ __forceinline__ void tile_frame_lanes(const FrameConst& fc, const SphereSet& S, const GroomView& g,
                                                  uint32_t tile, float4* s_p, float4* s_v, TileStats* s_ts) {
   static_assert(K == 2 || K == 4 || K == 8 || K == 16, "lane groups of 2, 4, 8 or 16");

@@ -560,6 +560,10 @@ __device__ __forceinline__ bool flagged(const SphereFilter<NF>& F, V3 w) {
   return m <= -dot(w, w);
 }
 
+// Spheres of a groom up to which its strands reach few of them, and the
+// push-out goes through all of those (measured at 7 and 16: push_seg).
+constexpr int kFewSpheres = 8;
+
 // The exact in-order push-out (push_out) of point j at its chain position w,
 // against the strand's reachable spheres in index order, read from shared
 // memory. A push by g moves D_j and s_j by +g and the next segment by -g
