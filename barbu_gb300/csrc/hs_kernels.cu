@@ -71,7 +71,8 @@ struct PlainVsmem {
 // spill 88 bytes), so that 11 blocks fit an SM rather than 10: 100,003
 // strands x 8 alone 26.5 -> 21.2 us (their 1,563 blocks are then one wave),
 // three such grooms in turn 14.9 -> 14.4 us.
-template <int CAP, bool REF, bool FAST>
+// MANY: the DFTL push-out among many spheres (strand_frame_regs_dftl).
+template <int CAP, bool REF, bool FAST, bool MANY>
 __global__ void __launch_bounds__(kStepBlock, REF ? 11 : 0) k_step(GroomView g, FrameConst fc) {
   extern __shared__ float4 s_vel[];  // per-thread velocity rows, when in shared memory
   __shared__ float4 s_c[HS_MAX_SPHERES];
@@ -82,14 +83,15 @@ __global__ void __launch_bounds__(kStepBlock, REF ? 11 : 0) k_step(GroomView g, 
   frame_acquire();
   const uint32_t s = blockIdx.x * kStepBlock + threadIdx.x;
   if constexpr (REF) strand_frame_ref<CAP, PlainVsmem<CAP>::value>(fc, S, g, s, s < g.nstrands, s_vel, threadIdx.x);
-  else strand_frame_regs_dftl<CAP, PlainVsmem<CAP>::value, FAST>(fc, S, g, s, s < g.nstrands, s_vel, threadIdx.x);
+  else
+    strand_frame_regs_dftl<CAP, PlainVsmem<CAP>::value, FAST, MANY>(fc, S, g, s, s < g.nstrands, s_vel, threadIdx.x);
 }
 
-template <int CAP, bool REF, bool FAST>
+template <int CAP, bool REF, bool FAST, bool MANY = false>
 cudaError_t launch_step_cap(const GroomView& g, const FrameConst& fc, cudaStream_t st) {
   const unsigned grid = (g.nstrands + kStepBlock - 1) / kStepBlock;
   const size_t smem = PlainVsmem<CAP>::value ? vslot_bytes<CAP>(kStepBlock) : 0;
-  return launch_overlapped(k_step<CAP, REF, FAST>, grid, kStepBlock, smem, st, g, fc);
+  return launch_overlapped(k_step<CAP, REF, FAST, MANY>, grid, kStepBlock, smem, st, g, fc);
 }
 
 bool fast_frame(const FrameConst& fc) { return fc.mode == HS_MODE_DFTL && fc.contract == HS_CONTRACT_FAST; }
@@ -97,6 +99,9 @@ bool fast_frame(const FrameConst& fc) { return fc.mode == HS_MODE_DFTL && fc.con
 template <int CAP>
 cudaError_t launch_step_mode(const GroomView& g, const FrameConst& fc, cudaStream_t st) {
   if (fc.mode == HS_MODE_REFERENCE) return launch_step_cap<CAP, true, false>(g, fc, st);
+  if (fc.nspheres > kFewSpheres)
+    return fast_frame(fc) ? launch_step_cap<CAP, false, true, true>(g, fc, st)
+                          : launch_step_cap<CAP, false, false, true>(g, fc, st);
   return fast_frame(fc) ? launch_step_cap<CAP, false, true>(g, fc, st) : launch_step_cap<CAP, false, false>(g, fc, st);
 }
 

@@ -578,8 +578,9 @@ constexpr int kFewSpheres = 8;
 // no other). 262,144 x 32 strands among 16 spheres: 241 -> 231 us a frame
 // (EXACT), 215 -> 211 us (FAST); the code is larger, which costs the
 // batched kernel more than it saves (64 grooms: 782 -> 824 us) and grooms
-// among few spheres (the 7 above: 49.6 -> 52.1 us).
-template <bool PICK, bool FAST, int NF>
+// among few spheres (the 7 above: 49.6 -> 52.1 us). BRANCH: past the spheres
+// that the point is not inside, where it goes through many.
+template <bool PICK, bool FAST, bool BRANCH = false, int NF>
 __device__ __forceinline__ void push_seg(const SphereFilter<NF>& F, const SphereSet& S, V3 w, V3& D, V3& s, V3& s_next,
                                          bool tip) {
   uint32_t todo = F.reach;
@@ -606,6 +607,7 @@ __device__ __forceinline__ void push_seg(const SphereFilter<NF>& F, const Sphere
     const V3 d = sub(p, cc);
     const float d2 = dot(d, d);
     const bool hit = d2 < S.r2[k];
+    if (BRANCH && !hit) continue;
     const V3 u = mul(d, FAST ? rsqrt_fast(d2) : inversesqrt(d2));
     const bool off = d2 > 0.0f;  // not at the centre
     const V3 q = add(cc, mul(c.w, v3(off ? u.x : 0.0f, off ? u.y : 1.0f, off ? u.z : 0.0f)));
@@ -1341,7 +1343,13 @@ __device__ __forceinline__ void strand_frame_stream(const FrameConst& fc, const 
 // shared rows (VStore, hs_step.cuh). The passes of substep_multi_pass_seg,
 // unrolled over CAP; with one iteration they compute what
 // substep_single_pass_seg does, operation for operation.
-template <int CAP, bool VSMEM, bool FAST = false>
+// MANY (more than kFewSpheres spheres): the push-out branches past spheres
+// the point is not inside. Registers are for four filter slots, so a strand
+// that reaches more sends most points through all of them: 50,021 x 8 among
+// 32 spheres, 8 substeps, EXACT, 47.8 -> 40.1 us, x 4 22.6 -> 18.6; among 12
+// 21.4 -> 20.6. (Eight slots and flagged spheres only take 36.4 there, but 43
+// against 37 us for 120,000 x 8 among 24.)
+template <int CAP, bool VSMEM, bool FAST, bool MANY>
 __device__ __forceinline__ void strand_frame_regs_dftl(const FrameConst& fc, const SphereSet& S, const GroomView& g,
                                                        uint32_t s, bool active, float4* vs_rows, int thread) {
   const int n = static_cast<int>(g.npoints);
@@ -1424,7 +1432,7 @@ __device__ __forceinline__ void strand_frame_regs_dftl(const FrameConst& fc, con
           if (i >= 2) {
             const bool tip = i == n;
             V3 Dj = D_prev, sj = s_prev;
-            if (flagged(F, w_prev)) push_seg<false, FAST>(F, S, w_prev, Dj, sj, sn, tip);
+            if (flagged(F, w_prev)) push_seg<false, FAST, MANY>(F, S, w_prev, Dj, sj, sn, tip);
             const V3 out = last_it ? vel_of(K, tip ? Dj : fmas(K.neg_damping, e, Dj)) : Dj;
             Sg[i - 1] = sj;
             vs.set(i - 1, f4(out, rest_prev));
