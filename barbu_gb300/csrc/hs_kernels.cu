@@ -180,30 +180,53 @@ size_t tmem_step_smem(uint32_t npoints) {
 }
 
 // Pairs of substeps a DFTL groom runs at once. They pay where schedulers wait
-// on chain links: less than a wave of warps (16 an SM, 8 for more than 32
-// points), longer strands, sphere tests to run two-wide. Single pass against
-// one pair / two pairs, us a frame, 8 substeps (EXACT; FAST gains a few percent
-// less):
-//   less than a wave  60,000 x 32 among 7 spheres 48.5 / 42.8, among 32 126 /
-//                     93; 60,000 x 16 among 24 48.9 / 42.0; 50,021 x 12 among
-//                     7 16.5 / 17.2, x 23 with two exports (S 5) 37.3 / 37.8;
-//                     38,133 x 32 without 10.8 / 11.9 (S 4);
-//                     20,000 x 36 among 8 47.7 / 35.5 / 36.6
-//   more              262,144 x 32 among 7 125 / 131; 150,000 x 36 among 4 111
-//                     / 113 / 117; 150,000 x 64 among 4 180 / 175 / 172, among
-//                     32 401 / 392 / 343
-//   one sphere        60,000 x 32 (FAST) 37.1 / 37.7; 150,000 x 64 253 / 225 /
-//                     229 (a head: every strand is near it)
-//   none              150,000 x 36 97 / 103 / 104, x 64 159 / 159 / 153
+// on chain links, and where sphere tests run two-wide: less than a wave of
+// warps (16 an SM, 8 for more than 32 points), longer strands, more spheres.
+// Among more than 8 spheres one substep at a time goes through flagged spheres
+// only (push_seg), which pairs do not: among 11 to 16 that is the faster form
+// up to 32 points; further on pairs pay again, more and more. An odd substep
+// is left over and changes form: it takes the gain away but for the most
+// spheres. Grooms in turn on streams of their own share the SMs, one alone
+// does not: the lines lie where both gain, or one gains and the other loses
+// less. Single pass against one pair / two pairs, us a frame, 8 substeps
+// unless S is given (EXACT; three grooms in turn, hair settled among the
+// spheres):
+//   half a wave       23,347 x 24 among 7 spheres 31.8 / 29.6 (FAST 27.6 /
+//                     27.0), x 28 (S 5) 33.1 / 27.5; among 12 33.1 / 38.0,
+//                     among 24 84.7 / 62.0; x 16 among 32 70.8 / 47.6
+//   a wave            76,267 x 24 among 7 48.9 / 50.1, among 24 82.2 / 94.0;
+//                     x 28 (S 5) among 7 40.7 / 49.8, among 16 47.4 / 70.3; x
+//                     32 among 32 217 / 165, S 5 126 / 128; 50,585 x 23 among
+//                     7 (S 5) 33.0 / 32.7
+//   more than 32      25,292 x 36 among 4 33.1 / 31.9 / 32.1, x 64 59.6 / 55.2
+//     points          / 53.6; 11,673 x 64 among 12 (S 5) 45.5 / 63.2 / 51.9;
+//                     116,736 x 36 among 4 123 / 123 / 129, among 16 166 / 195
+//                     / 164, among 24 (S 5) 192 / 256 / 215; x 64 among 4 (S
+//                     5) 151 / 154 / 160, among 32 717 / 687 / 567, S 5 461 /
+//                     481 / 423
+//   one sphere        x 64 315 / 275 / 282 (a head: every strand is near it);
+//                     50,585 x 32 53.7 / 53.1
+//   none              x 64 176 / 169 / 158; 25,292 x 36 22.6 / 24.3 / 23.5
 int step_pairs(const GroomView& g, const FrameConst& fc) {
   if (fc.iterations != 1 || fc.substeps < 2) return 0;
-  const bool is_long = g.npoints > 32;
   const uint32_t sms = static_cast<uint32_t>(device_attribute(cudaDevAttrMultiProcessorCount, 152));
-  const bool wave = (g.nstrands + 31) / 32 <= (is_long ? 8u : 16u) * sms;
-  if (!is_long) return wave && fc.nspheres > 1 && (g.npoints > 24 || fc.nspheres > 16) ? 1 : 0;
-  if (fc.nspheres == 0) return g.npoints > 48 ? 2 : 0;
-  if (fc.nspheres == 1 || wave) return 1;
-  return fc.nspheres > 8 || g.npoints > 48 ? 2 : 0;
+  const uint32_t tiles = (g.nstrands + 31) / 32;
+  const int spheres = fc.nspheres;
+  const bool even = fc.substeps % 2 == 0;
+  const bool half = tiles <= 8u * sms;  // half a wave up to 32 points, a wave above
+  if (g.npoints > 32) {
+    if (spheres == 0) return g.npoints > 48 ? 2 : 0;
+    if (spheres == 1) return 1;
+    if (spheres <= kFewSpheres) return half ? 1 : (even && g.npoints > 48 ? 2 : 0);
+    return even || spheres <= 12 || spheres > 24 || g.npoints > 48 ? 2 : 0;
+  }
+  const bool most = tiles <= 12u * sms, wave = tiles <= 16u * sms, fast = fast_frame(fc);
+  if (!even) return spheres > 24 && most && g.npoints >= (half ? 12u : 16u) ? 1 : 0;
+  if (spheres > 24) return wave && g.npoints >= 12 ? 1 : 0;
+  if (spheres > 20) return most && g.npoints >= 16 ? 1 : 0;
+  if (g.npoints < 20 || !(fast ? half : most)) return 0;
+  if (spheres > 16) return half && !fast ? 1 : 0;
+  return spheres >= (fast ? 6 : 4) && spheres <= 10 ? 1 : 0;
 }
 
 using StepKernel = void (*)(GroomView, FrameConst);
