@@ -95,14 +95,12 @@ struct SphereCache {
   float2 ncx[M / 2], ncy[M / 2], ncz[M / 2];  // negated centres, in pairs
   int ncached;      // spheres cached (this lane's)
   uint32_t rest;    // reachable spheres beyond the cached ones, in index order
-  uint32_t reach;   // every reachable sphere
 };
 
 template <int M>
 __device__ __forceinline__ SphereCache<M> cache_spheres(const SphereSet& S, uint32_t reach) {
   SphereCache<M> C;
   C.ncached = 0;
-  C.reach = reach;
 #pragma unroll
   for (int q = 0; q < M; ++q) {
     C.cx[q] = C.cy[q] = C.cz[q] = C.r[q] = 0.0f;
@@ -129,21 +127,17 @@ __device__ __forceinline__ SphereCache<M> cache_spheres(const SphereSet& S, uint
   return C;
 }
 
-// CollideSphere(+1, c, r, p) (cs_simulation.glsl:129-139) of one sphere;
-// true if the sphere pushed the point. FAST: the normal's reciprocal
-// square root is the hardware's (the FAST contract, DFTL mode only).
-template <bool REF, bool FAST = false>
-__device__ __forceinline__ bool push_out(V3 cc, float r, float r2, V3& p, V3& v) {
-  static_assert(!(REF && FAST), "reference mode has the EXACT contract only");
+// CollideSphere(+1, c, r, p) (cs_simulation.glsl:129-139) of one sphere. VEL:
+// the point's velocity is reflected too (a substep's last iteration).
+template <bool VEL>
+__device__ __forceinline__ void push_out(V3 cc, float r, float r2, V3& p, V3& v) {
   const V3 pt = sub(p, cc);
   const float dp = dot(pt, pt);
   if (dp < r2) {
-    const V3 nn = dp > 0.0f ? mul(pt, FAST ? rsqrt_fast(dp) : inversesqrt(dp)) : v3(0.0f, 1.0f, 0.0f);
+    const V3 nn = dp > 0.0f ? mul(pt, inversesqrt(dp)) : v3(0.0f, 1.0f, 0.0f);
     p = add(cc, mul(r, nn));
-    if (REF) v = reflect(v, nn);  // :137
-    return true;
+    if (VEL) v = reflect(v, nn);  // :137
   }
-  return false;
 }
 
 // Collision of one point, split so the cheap part can be scheduled with
@@ -177,26 +171,22 @@ __device__ __forceinline__ bool tests(const SphereCache<M>& C, V3 p) {
 
 // The exact in-order push-out (rare), kept inline: an out-of-line call
 // would take the addresses of the callers' per-lane arrays and move them
-// to local memory. True if any sphere pushed the point.
-template <bool REF, int NC, int M>
-__device__ __forceinline__ bool push_all(const SphereCache<M>& C, const SphereSet& S, V3& p, V3& v) {
-  bool pushed = false;
+// to local memory.
+template <bool VEL, int NC, int M>
+__device__ __forceinline__ void push_all(const SphereCache<M>& C, const SphereSet& S, V3& p, V3& v) {
 #pragma unroll
   for (int q = 0; q < M; ++q)
-    if (q < C.ncached) pushed |= push_out<REF>(v3(C.cx[q], C.cy[q], C.cz[q]), C.r[q], C.r2[q], p, v);
-  uint32_t more = C.rest;
-  while (more) {
+    if (q < C.ncached) push_out<VEL>(v3(C.cx[q], C.cy[q], C.cz[q]), C.r[q], C.r2[q], p, v);
+  for (uint32_t more = C.rest; more; more &= more - 1u) {
     const int k = __ffs(more) - 1;
-    more &= more - 1u;
     const float4 c = S.c[k];
-    pushed |= push_out<REF>(v3(c.x, c.y, c.z), c.w, S.r2[k], p, v);
+    push_out<VEL>(v3(c.x, c.y, c.z), c.w, S.r2[k], p, v);
   }
-  return pushed;
 }
 
-template <bool REF, int NC, int M>
+template <bool VEL, int NC, int M>
 __device__ __forceinline__ void collide_fast(const SphereCache<M>& C, const SphereSet& S, V3& p, V3& v) {
-  if (tests<NC>(C, p)) push_all<REF, NC>(C, S, p, v);
+  if (tests<NC>(C, p)) push_all<VEL, NC>(C, S, p, v);
 }
 
 // Per-strand constants of a frame.
@@ -204,7 +194,6 @@ struct StrandConsts {
   V3 F;            // force per unit mass
   V3 h2F;          // h^2 F (DFTL: the force's part of a substep's displacement)
   float h, h2, inv_h, damping, neg_damping, lscale;
-  bool fast;       // DFTL chain links under the FAST contract (hs_contract)
 };
 
 // ---- reference mode: world coordinates (cs_simulation.glsl) -----------
@@ -1112,7 +1101,6 @@ __device__ __forceinline__ StrandConsts strand_consts(const FrameConst& fc, cons
   K.damping = fc.damping;
   K.neg_damping = -fc.damping;
   K.lscale = fc.length_scale;
-  K.fast = fc.contract == HS_CONTRACT_FAST;
   return K;
 }
 
