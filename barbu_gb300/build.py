@@ -1,7 +1,8 @@
 """Build the hair-simulation library in tree.
 
 barbu_gb300/csrc/*.cu -> barbu_gb300/lib/libhairsim.so, for sm_103a only, and
-the binding's call module, csrc/hs_pycalls.c -> barbu_gb300/_hscalls.so.
+the binding's call module, csrc/hs_pycalls.c -> barbu_gb300/_hscalls<suffix>,
+the suffix of this interpreter (its ABI).
 One nvcc process per translation unit, in parallel, then one link. Host code
 is compiled without floating-point contraction so host-side parameter
 arithmetic rounds like the device's.
@@ -21,7 +22,7 @@ CSRC = os.path.join(HERE, "csrc")
 BUILD = os.path.join(HERE, "_build")
 LIB_DIR = os.path.join(HERE, "lib")
 LIB = os.path.join(LIB_DIR, "libhairsim.so")
-CALLS = os.path.join(HERE, "_hscalls.so")
+CALLS = os.path.join(HERE, "_hscalls" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 
 
@@ -49,15 +50,25 @@ def _compile(src: str, verbose_ptxas: bool) -> str:
     return obj
 
 
-def build_calls() -> str:
+def build_calls() -> str | None:
+    """The binding's call module, or None (and a line on stderr) where it cannot
+    be compiled, without a C compiler or Python.h: the binding then makes every
+    call through ctypes."""
     tmp = CALLS + ".tmp"
     cmd = [shutil.which("gcc") or "cc", "-O2", "-fPIC", "-shared", "-fvisibility=hidden", "-Wall", "-I",
            sysconfig.get_paths()["include"], os.path.join(CSRC, "hs_pycalls.c"), "-o", tmp]
-    r = subprocess.run(cmd, capture_output=True, text=True)
-    if r.returncode != 0:
-        raise RuntimeError(f"building {CALLS} failed:\n{r.stdout}\n{r.stderr}")
-    os.replace(tmp, CALLS)
-    return CALLS
+    try:
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        failed = None if r.returncode == 0 else (r.stderr.strip().splitlines() or ["compiler error"])[0]
+    except OSError as e:
+        failed = str(e)
+    if failed is None:
+        os.replace(tmp, CALLS)
+        return CALLS
+    sys.stderr.write(f"{os.path.basename(CALLS)} not built, calls go through ctypes: {failed}\n")
+    if os.path.exists(CALLS):  # of older sources
+        os.remove(CALLS)
+    return None
 
 
 def build(verbose_ptxas: bool = False) -> str:
@@ -71,8 +82,8 @@ def build(verbose_ptxas: bool = False) -> str:
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
-    os.replace(tmp, LIB)
     build_calls()
+    os.replace(tmp, LIB)
     return LIB
 
 

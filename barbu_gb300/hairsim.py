@@ -101,6 +101,17 @@ def _declare(L):
         fn.argtypes = args
 
 
+class _CtypesCalls:
+    """The call module's functions where it has not been built (for this
+    interpreter): they take nothing, and every call goes the general way."""
+
+    @staticmethod
+    def frame(*args):
+        return None
+
+    floats = rows = frame
+
+
 def lib():
     """Loads libhairsim.so (raises if it has not been built)."""
     global _lib, _calls
@@ -108,12 +119,15 @@ def lib():
         if not os.path.exists(LIB_PATH):
             raise ImportError(f"{LIB_PATH} is missing: build it with `python -m barbu_gb300.build` "
                               "(the library has no CPU fallback)")
-        from . import _hscalls  # built with the library
+        try:
+            from . import _hscalls as calls  # built with the library
+        except ImportError:
+            calls = _CtypesCalls
         L = C.CDLL(LIB_PATH)
         _declare(L)
         for name in _ADDRESS:
             _ADDRESS[name] = C.cast(getattr(L, name), C.c_void_p).value
-        _calls = _hscalls
+        _calls = calls
         _lib = L
     return _lib
 
