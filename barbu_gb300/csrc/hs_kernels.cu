@@ -504,6 +504,10 @@ int plain_mapping(const GroomView& g, const FrameConst& fc, int mapping) {
   // 65.4 / 45.0, 54,476 x 32 without spheres (44.8) 31.0 / 17.4. A group of
   // two holds few warps of long strands in shared memory, and gains only while
   // they are resident together (22,431 x 64, S 2: 27.3 / 19.7).
+  // The multiples lie between those of one groom alone (3.5, 6.5, 9.5 and 13 by
+  // the same classes) and of three in turn on streams of their own, which share
+  // the SMs (1.9, 3.3, 4.3 and 6.4): 12,000 x 16 among 2, S 5, FAST, takes 18.6
+  // / 22.8 alone, 13.6 / 9.2 in turn.
   const uint32_t N = g.npoints, S = static_cast<uint32_t>(fc.substeps);
   const float multiple = fc.nspheres > 8 ? 8.5f : fc.nspheres > 1 ? 7.0f : fc.nspheres == 1 || N <= 8 ? 5.0f : 3.0f;
   float limit = multiple * static_cast<float>(S * N) / static_cast<float>(N + 2 * S);
